@@ -2,12 +2,14 @@
 // programs replayed through CUDA graphs, and FP64 reductions.
 #include "../../include/cast_b200.h"
 #include "internal.hpp"
+#include "pass_plan.hpp"
 
 #include <algorithm>
 
 #include <exception>
 #include <map>
 #include <mutex>
+#include <set>
 #include <utility>
 
 using cb2::clear_err;
@@ -54,18 +56,45 @@ struct Program {
   bool split = false;  // complex64 gates with 4..6 qubits run on the tensor cores
   std::vector<GateData> gates;
   std::map<std::pair<uint64_t, void *>, cudaGraphExec_t> graphs;
+  std::set<std::pair<uint64_t, void *>> ran;  // (statevector, stream) pairs run once
+  // How the gates are grouped into passes, newest last.  A changed kernel choice
+  // makes a new plan; graphs captured from an older one still read its matrices,
+  // so it stays until the graphs go.
+  std::vector<cb2::PassPlan *> plans;
+  uint32_t plan_epoch = 0;  // kernel choices the newest plan was made under
   std::mutex mu;
 
   ~Program() {
-    for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+    drop_graphs();
     for (auto &g : gates) cb2::free_gate_device(g);
   }
 
   void drop_graphs() {
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
+    ran.clear();
+    for (cb2::PassPlan *p : plans) cb2::free_pass_plan(p);
+    plans.clear();
   }
 
+  bool ensure_plan(std::string &err) {
+    const uint32_t epoch = cb2::gate_choice_epoch();
+    if (plans.empty() || plan_epoch != epoch) {
+      cb2::PassPlan *p = cb2::make_pass_plan(gates, n);
+      plans.push_back(p);
+      plan_epoch = epoch;
+    }
+    return cb2::upload_pass_plan(*plans.back(), err);
+  }
+
+  bool mark_plans(cudaStream_t s, std::string &err) {
+    for (cb2::PassPlan *p : plans)
+      if (!cb2::mark_pass_plan(*p, s, err)) return false;
+    return true;
+  }
+
+  // Gate after gate, each on its own kernel: for a stream that is being captured,
+  // where nothing may be allocated and a caller's graph may outlive this program.
   bool launch_all(uint64_t sv, cudaStream_t s, std::string &err) {
     for (auto &g : gates)
       if (!cb2::launch_gate(g, reinterpret_cast<void *>(sv), n, s, err)) return false;
@@ -316,6 +345,29 @@ uint32_t cast_b200_program_num_gates(const void *program) {
   return p && p->magic == kProgramMagic ? (uint32_t)p->gates.size() : 0;
 }
 
+int cast_b200_program_plan(void *program, uint32_t *out_pass, uint32_t *out_place, char *err_buf,
+                           size_t err_buf_len) {
+  Program *p = as_program(program);
+  if (!p) {
+    write_err(err_buf, err_buf_len, "invalid program handle");
+    return -1;
+  }
+  try {
+    std::lock_guard<std::mutex> lock(p->mu);
+    const std::vector<cb2::Pass> passes = cb2::program_passes(p->gates, p->n);
+    for (uint32_t i = 0; i < passes.size(); ++i)
+      for (uint32_t j = 0; j < passes[i].gates.size(); ++j) {
+        if (out_pass) out_pass[passes[i].gates[j]] = i;
+        if (out_place) out_place[passes[i].gates[j]] = j;
+      }
+    clear_err(err_buf, err_buf_len);
+    return (int)passes.size();
+  } catch (const std::exception &ex) {
+    write_err(err_buf, err_buf_len, ex.what());
+    return -1;
+  }
+}
+
 int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use_graph,
                           char *err_buf, size_t err_buf_len) {
   Program *p = as_program(program);
@@ -334,15 +386,33 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
     std::lock_guard<std::mutex> lock(p->mu);
     std::string err;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (!use_graph || !s || p->gates.empty()) {
-      if (!p->launch_all(sv_dptr, s, err)) {
+    // merged passes, or gate after gate where nothing may be allocated (a stream
+    // under capture) or nothing could be
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const bool may_plan = cudaStreamIsCapturing(s, &capturing) == cudaSuccess &&
+                          capturing == cudaStreamCaptureStatusNone && !p->gates.empty();
+    const bool plain = !may_plan || !p->ensure_plan(err);
+    if (plain) {
+      cudaGetLastError();
+      err.clear();
+    }
+    void *sv = reinterpret_cast<void *>(sv_dptr);
+    const auto key = std::make_pair(sv_dptr, stream);
+    // The first run on a (statevector, stream) pair launches directly: capturing
+    // and instantiating a graph costs more than the launches it replays, which a
+    // program that runs once (Simulator.simulate) would pay for nothing.
+    const bool first = !plain && use_graph && s && p->graphs.find(key) == p->graphs.end() &&
+                       p->ran.insert(key).second;
+    if (!use_graph || !s || p->gates.empty() || first) {
+      if (!(plain ? p->launch_all(sv_dptr, s, err)
+                  : cb2::launch_pass_plan(*p->plans.back(), p->gates, sv, p->n, s, err) &&
+                        p->mark_plans(s, err))) {
         write_err(err_buf, err_buf_len, err);
         return 1;
       }
       clear_err(err_buf, err_buf_len);
       return 0;
     }
-    auto key = std::make_pair(sv_dptr, stream);
     auto it = p->graphs.find(key);
     if (it == p->graphs.end()) {
       cudaGraph_t graph = nullptr;
@@ -352,7 +422,8 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
         write_err(err_buf, err_buf_len, err);
         return 1;
       }
-      const bool launched = p->launch_all(sv_dptr, s, err);
+      const bool launched = plain ? p->launch_all(sv_dptr, s, err)
+                                  : cb2::launch_pass_plan(*p->plans.back(), p->gates, sv, p->n, s, err);
       const cudaError_t end_rc = cudaStreamEndCapture(s, &graph);
       if (!launched || !cuda_ok(end_rc, "cudaStreamEndCapture", err) ||
           !cuda_ok(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate", err)) {
@@ -363,7 +434,7 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
       cudaGraphDestroy(graph);
       it = p->graphs.emplace(key, exec).first;
     }
-    if (!cuda_ok(cudaGraphLaunch(it->second, s), "cudaGraphLaunch", err)) {
+    if (!cuda_ok(cudaGraphLaunch(it->second, s), "cudaGraphLaunch", err) || !p->mark_plans(s, err)) {
       write_err(err_buf, err_buf_len, err);
       return 1;
     }

@@ -957,6 +957,7 @@ struct KernelChoice {
   std::atomic<int> tile_bits{0};
 };
 KernelChoice g_choice[2][5][32];
+std::atomic<uint32_t> g_choice_epoch{0};
 
 bool tile_chosen(const GateData &g, uint32_t n, TileArgs &a) {
   if (g.k > 4) return false;
@@ -1016,7 +1017,13 @@ bool launch_t(const GateData &g, void *sv, uint32_t n, const Targets &t, cudaStr
 
 }  // namespace
 
-int set_gate_path(int path) { return g_gate_path.exchange(path < 0 || path > 2 ? 0 : path); }
+uint32_t gate_choice_epoch() { return g_choice_epoch.load(); }
+
+int set_gate_path(int path) {
+  const int prev = g_gate_path.exchange(path < 0 || path > 2 ? 0 : path);
+  ++g_choice_epoch;
+  return prev;
+}
 
 bool set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int engine,
                        uint32_t tile_bits_, std::string &err) {
@@ -1030,7 +1037,17 @@ bool set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int eng
   KernelChoice &c = g_choice[precision][k][low_mask];
   c.engine.store(engine);
   c.tile_bits.store((int)tile_bits_);
+  ++g_choice_epoch;
   return true;
+}
+
+bool gate_choice_forced(const GateData &g) {
+  if (gate_path_override() != 0) return true;
+  if (g.k > 4) return false;
+  uint32_t low_bits = 0;
+  for (uint32_t b = 0; b < g.k; ++b)
+    if (g.qubits[b] < 5) low_bits |= 1u << g.qubits[b];
+  return low_bits && g_choice[g.precision ? 1 : 0][g.k][low_bits].engine.load(std::memory_order_relaxed) >= 0;
 }
 
 int sm_count() {

@@ -105,6 +105,26 @@ bool set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int eng
                        uint32_t tile_bits, std::string &err);
 bool upload_gate_matrix(GateData &g, std::string &err);  // fills g.d_mat
 
+// True while a kernel choice set from outside (a forced path or an autotuned
+// class) decides how this gate runs; such gates are not merged into passes.
+bool gate_choice_forced(const GateData &g);
+uint32_t gate_choice_epoch();  // changes whenever such a choice is set
+
+// Merged passes (gate_pass.cu): a program's gates grouped into passes over the
+// statevector.  make_pass_plan touches no device; upload_pass_plan puts the
+// matrices on the device (synchronous, not under stream capture);
+// launch_pass_plan enqueues every pass; mark_pass_plan records, behind launches
+// on `s`, that the plan's device memory is in use until then.
+struct Pass;
+struct PassPlan;
+std::vector<Pass> program_passes(const std::vector<GateData> &gates, uint32_t n);
+PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n);
+void free_pass_plan(PassPlan *p);
+bool upload_pass_plan(PassPlan &p, std::string &err);
+bool launch_pass_plan(PassPlan &p, const std::vector<GateData> &gates, void *sv, uint32_t n,
+                      cudaStream_t s, std::string &err);
+bool mark_pass_plan(PassPlan &p, cudaStream_t s, std::string &err);
+
 // Reductions (reduce_kernels.cu): synchronous on `s`, except scale (enqueued).
 bool norm_squared(const void *x, uint64_t n_scalars, uint8_t precision, double *out,
                   cudaStream_t s, std::string &err);

@@ -116,6 +116,16 @@ class GateProgram:
     def __len__(self):
         return int(L.lib().cast_b200_program_num_gates(self.handle))
 
+    def plan(self) -> tuple[np.ndarray, np.ndarray]:
+        """(pass, place in the pass) of every gate: how ``run`` groups them
+        (cast_b200_program_plan; touches no device)."""
+        out = np.zeros((2, max(1, len(self))), dtype=np.uint32)
+        eb = L.errbuf()
+        if L.lib().cast_b200_program_plan(self.handle, out[0].ctypes.data_as(L.c_u32p),
+                                          out[1].ctypes.data_as(L.c_u32p), eb, L.ERR_LEN) < 0:
+            raise RuntimeError(f"program_plan failed: {eb.value.decode()}")
+        return out[0, :len(self)], out[1, :len(self)]
+
     def run(self, sv: CudaStatevector, stream: Stream | None = None, use_graph: bool = True) -> None:
         if sv.n_qubits() != self.n_qubits or sv.precision() != self.precision:
             raise ValueError("statevector does not match the program")

@@ -92,7 +92,11 @@ int cast_b200_gate_engine(uint8_t precision, uint32_t sv_n_qubits, const cast_co
  * once and replayed many times: the device-side analogue of the reference's
  * compile_batch + apply-all + sync loop (src/simulator/mod.rs:523-562,
  * src/simulator/bench.rs:136-167).  With use_graph != 0 the launches are
- * captured once per (statevector, stream) into a CUDA graph and replayed. */
+ * captured into a CUDA graph at the second run on a (statevector, stream) pair
+ * and replayed from then on.  Neighbouring dense gates of up to 4 qubits may
+ * share one pass over the state (gates that share a qubit keep their order,
+ * gates on disjoint qubits may swap); on a stream under capture by the caller,
+ * and while a kernel choice is forced, every gate runs on its own kernel. */
 void *cast_b200_program_create(uint8_t precision, uint32_t sv_n_qubits, double ztol, double otol,
                                char *err_buf, size_t err_buf_len);
 int cast_b200_program_add_gate(void *program, const cast_complex64_t *matrix,
@@ -117,6 +121,12 @@ int cast_b200_tensor_status(uint32_t *out_bits, char *err_buf, size_t err_buf_le
  * mode. */
 int cast_b200_set_tensor_loader(int mode);
 uint32_t cast_b200_program_num_gates(const void *program);
+/* How program_run groups the gates: out_pass[i] is gate i's pass and
+ * out_place[i] its place in that pass (either may be NULL; num_gates entries).
+ * Returns the number of passes, -1 on an error; touches no device.  A gate alone
+ * in its pass runs on the kernel cast_b200_gate_engine names. */
+int cast_b200_program_plan(void *program, uint32_t *out_pass, uint32_t *out_place, char *err_buf,
+                           size_t err_buf_len);
 int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use_graph,
                           char *err_buf, size_t err_buf_len);
 void cast_b200_program_destroy(void *program);

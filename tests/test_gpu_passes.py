@@ -1,0 +1,53 @@
+"""Merged gate passes (several gates of a program for one read and one write of
+the state) against the oracle, at the edges of their tiles."""
+import numpy as np
+import pytest
+
+from cast_simulator_b200 import types as T
+from cast_simulator_b200.cuda import CudaPrecision, CudaStatevector
+from cast_simulator_b200.simulator import GateProgram, Stream
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _random_gates(n, count, widths, seed):
+    rng = np.random.default_rng(seed)
+    out = []
+    for i in range(count):
+        k = min(n, widths[i % len(widths)])
+        qs = rng.choice(n, size=k, replace=False)
+        if i % 3 == 0:  # neighbouring targets, the common shape of fused circuits
+            q0 = int(rng.integers(0, n - k + 1))
+            qs = np.arange(q0, q0 + k)
+        out.append(T.QuantumGate.random_unitary([int(q) for q in qs], rng))
+    return out
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("n,widths", [
+    (6, (2, 3)),           # below the smallest tile: one kernel a gate
+    (7, (1, 2, 3, 4)),     # one tile, one block a gate
+    (8, (4,)), (9, (1, 2)), (11, (3,)),
+    (12, (1, 2, 3, 4)), (13, (4, 3)), (16, (2, 4)), (19, (4, 3, 1)), (20, (1, 2, 3, 4)),
+    (22, (4, 3)),          # complex64: 4-qubit gates alone, 3-qubit ones merged
+])
+@pytest.mark.parametrize("prec", [CudaPrecision.F64, CudaPrecision.F32])
+def test_program_matches_oracle(n, widths, graph, prec):
+    rng = np.random.default_rng(n)
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    psi /= np.linalg.norm(psi)
+    gates = _random_gates(n, 24, widths, 100 + n)
+    tol = 1e-12 if prec == CudaPrecision.F64 else 1e-6
+    prog = GateProgram(prec, n, tol, tol)
+    want = psi.copy()
+    for g in gates:
+        prog.add(g.matrix(), g.qubits())
+        O.apply_gate(want, g.matrix(), g.qubits())
+    sv, st = CudaStatevector(n, prec), Stream()
+    sv.upload(psi)
+    prog.run(sv, st, use_graph=graph)
+    st.sync()
+    # 24 unitary gates: each adds at most a few units of 2^k roundings
+    bound = 24 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
+    assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
