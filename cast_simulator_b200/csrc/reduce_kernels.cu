@@ -2,12 +2,13 @@
 //
 // Replaces src/cpp/cuda/cuda_kernels.cu of narix10yc/cast_simulator
 // (normSqPass1/2 at :124-167, scaleKernel at :171-196, C wrappers at :244-254).
-// Same two-pass structure - per-block FP64 partial sums over 128-bit loads into
-// a device scratch array, then one block folds the partials - but sized for
-// B200: 4 blocks of 256 threads per SM, 4 independent 128-bit loads in flight
-// per thread per iteration.  Both run on the legacy default stream, as the
-// reference's do (cuda_kernels.cu:236-238), so they order after earlier work on
-// blocking streams.
+// Per-block FP64 partial sums over 128-bit loads go into a device scratch array;
+// the launch's last block folds them in a fixed order and writes the result into
+// page-locked host memory.  One launch and one wait a call: the fold kernel and
+// the copy back that followed before took 27 of 29 us for a 16-qubit state.
+// cast_cuda_norm_squared and cast_cuda_scale run on the legacy default stream, as
+// the reference's do (cuda_kernels.cu:236-238), so they order after earlier work
+// on blocking streams.
 #include "../../include/ffi_cuda.h"
 #include "internal.hpp"
 
@@ -47,10 +48,50 @@ template <typename T> struct V16;
 template <> struct V16<float> { using type = float4; static constexpr int N = 4; };
 template <> struct V16<double> { using type = double2; static constexpr int N = 2; };
 
-// Pass 1: partial[blockIdx.x] = sum of squares of this block's share.
+// Blocks of the running launch that have written their partials.  One reduction
+// runs at a time (the scratch mutex) and its last block puts the count back to 0.
+__device__ unsigned g_blocks_done;
+
+// Called by every block once its partials are written: true in the block that
+// comes last, for which all partials are then visible.
+__device__ __forceinline__ bool last_block() {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(&g_blocks_done, 1u) == gridDim.x - 1;
+    if (last) g_blocks_done = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// out[c] = sum over blocks r of partial[r * cols + c], in a fixed order: the whole
+// block a column while they are few, else one warp a column.
+__device__ __forceinline__ void fold_columns(const double *partial, int rows, int cols, double *out) {
+  if (cols <= 2) {
+    for (int c = 0; c < cols; ++c) {
+      double v = 0;
+      for (int r = threadIdx.x; r < rows; r += kRedThreads) v += __ldcg(&partial[(size_t)r * cols + c]);
+      v = block_sum(v);
+      if (threadIdx.x == 0) out[c] = v;
+      __syncthreads();
+    }
+    return;
+  }
+  for (int c = threadIdx.x >> 5; c < cols; c += kRedThreads / 32) {
+    double v = 0;
+    for (int r = threadIdx.x & 31; r < rows; r += 32) v += __ldcg(&partial[(size_t)r * cols + c]);
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) out[c] = v;
+  }
+}
+
+// out[0] = sum of squares.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_norm_pass1(const T *__restrict__ x, uint64_t n,
-                                                           double *__restrict__ partial) {
+__global__ void __launch_bounds__(kRedThreads) k_norm(const T *__restrict__ x, uint64_t n, double *partial,
+                                                     double *__restrict__ out) {
   using V = typename V16<T>::type;
   constexpr int N = V16<T>::N;
   const V *xv = reinterpret_cast<const V *>(x);
@@ -74,15 +115,7 @@ __global__ void __launch_bounds__(kRedThreads) k_norm_pass1(const T *__restrict_
   }
   acc = block_sum(acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-}
-
-// Pass 2: out[0] = sum of the partials (one block).
-__global__ void __launch_bounds__(kRedThreads) k_norm_pass2(const double *__restrict__ partial,
-                                                            int n, double *__restrict__ out) {
-  double acc = 0;
-  for (int i = threadIdx.x; i < n; i += kRedThreads) acc += partial[i];
-  acc = block_sum(acc);
-  if (threadIdx.x == 0) out[0] = acc;
+  if (last_block()) fold_columns(partial, (int)gridDim.x, 1, out);
 }
 
 template <typename T>
@@ -104,34 +137,49 @@ __global__ void __launch_bounds__(kRedThreads) k_scale(T *__restrict__ x, uint64
   if (blockIdx.x == 0 && threadIdx.x < n - nv * N) x[nv * N + threadIdx.x] *= s;
 }
 
-// Scratch: partial sums + the final value, one buffer per device, allocated on
-// first use and grown on demand (the reference keeps the same kind of
-// process-wide scratch, cuda_kernels.cu:203-230).  The mutex serialises users
-// of the scratch.  Returns the current device's buffer, or null with a message.
+// Scratch of one device: per-block partials and a page-locked result buffer that
+// kernels write straight into.  Allocated on first use and grown on demand (the reference
+// keeps the same kind of process-wide scratch, cuda_kernels.cu:203-230).  The
+// mutex serialises its users, each until its result has arrived.
 std::mutex g_scratch_mu;
 constexpr int kMaxScratchDevices = 64;
-double *g_scratch_dev[kMaxScratchDevices] = {};
-int g_scratch_len[kMaxScratchDevices] = {};
+constexpr int kMaxResult = 4096;  // doubles: the largest marginal
+struct Scratch {
+  double *partial = nullptr;
+  int len = 0;
+  double *result = nullptr;  // page-locked, mapped
+};
+Scratch g_scratch_dev[kMaxScratchDevices];
 
-double *ensure_scratch(int len, std::string &err) {
+Scratch *ensure_scratch(int len, std::string &err) {
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return nullptr;
   if (dev < 0 || dev >= kMaxScratchDevices) {
     err = "reduction scratch: device index out of range";
     return nullptr;
   }
-  double *&p = g_scratch_dev[dev];
-  int &have = g_scratch_len[dev];
-  if (p && have >= len) return p;
-  if (p) cudaFree(p);
-  p = nullptr;
-  have = 0;
-  if (!cuda_ok(cudaMalloc(&p, sizeof(double) * len), "cudaMalloc (norm scratch)", err)) {
-    p = nullptr;
+  Scratch &s = g_scratch_dev[dev];
+  if (!s.result && !cuda_ok(cudaHostAlloc((void **)&s.result, sizeof(double) * kMaxResult,
+                                          cudaHostAllocMapped | cudaHostAllocPortable),
+                            "cudaHostAlloc (reduction result)", err)) {
+    s.result = nullptr;
     return nullptr;
   }
-  have = len;
-  return p;
+  if (s.partial && s.len >= len) return &s;
+  if (s.partial) cudaFree(s.partial);
+  s.partial = nullptr;
+  s.len = 0;
+  if (!cuda_ok(cudaMalloc((void **)&s.partial, sizeof(double) * len), "cudaMalloc (norm scratch)", err)) {
+    s.partial = nullptr;
+    return nullptr;
+  }
+  s.len = len;
+  return &s;
+}
+
+// Launch status, then the wait for the result in s.result.
+bool fetch_result(cudaStream_t stream, const char *what, std::string &err) {
+  return cuda_ok(cudaGetLastError(), what, err) && cuda_ok(cudaStreamSynchronize(stream), what, err);
 }
 
 unsigned red_grid(uint64_t nv) {
@@ -144,14 +192,12 @@ template <typename T>
 bool norm_sq_impl(const void *x, uint64_t n, double *out, cudaStream_t s, std::string &err) {
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   const unsigned grid = red_grid(n / V16<T>::N);
-  double *const g_scratch = ensure_scratch((int)grid + 1, err);
-  if (!g_scratch) return false;
-  k_norm_pass1<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, g_scratch);
-  k_norm_pass2<<<1, kRedThreads, 0, s>>>(g_scratch, (int)grid, g_scratch + grid);
-  if (!cuda_ok(cudaGetLastError(), "norm kernel launch", err)) return false;
-  return cuda_ok(cudaMemcpyAsync(out, g_scratch + grid, sizeof(double), cudaMemcpyDeviceToHost, s),
-                 "cudaMemcpyAsync (norm result)", err) &&
-         cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (norm)", err);
+  Scratch *const sc = ensure_scratch((int)grid, err);
+  if (!sc) return false;
+  k_norm<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->partial, sc->result);
+  if (!fetch_result(s, "norm", err)) return false;
+  *out = sc->result[0];
+  return true;
 }
 
 template <typename T>
@@ -162,118 +208,259 @@ bool scale_impl(void *x, uint64_t n, double scale, cudaStream_t s, std::string &
 }
 
 
-// <a|b> partials: (re, im) per block.
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_inner_pass1(const T *__restrict__ a,
-                                                            const T *__restrict__ b, uint64_t n_amps,
-                                                            double *__restrict__ partial) {
-  using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
-  const V *av = reinterpret_cast<const V *>(a);
-  const V *bv = reinterpret_cast<const V *>(b);
-  double re = 0, im = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * kRedThreads;
-  for (uint64_t i = (uint64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n_amps; i += stride) {
-    const V x = av[i], y = bv[i];
-    re += (double)x.x * y.x + (double)x.y * y.y;
-    im += (double)x.x * y.y - (double)x.y * y.x;
-  }
-  re = block_sum(re);
-  __syncthreads();
-  im = block_sum(im);
-  if (threadIdx.x == 0) {
-    partial[2 * blockIdx.x] = re;
-    partial[2 * blockIdx.x + 1] = im;
-  }
+// One 16-byte vector of a and b: 2 amplitudes in FP32, 1 in FP64.
+__device__ __forceinline__ void inner_add(float4 x, float4 y, double &re, double &im) {
+  re += (double)x.x * y.x + (double)x.y * y.y;
+  im += (double)x.x * y.y - (double)x.y * y.x;
+  re += (double)x.z * y.z + (double)x.w * y.w;
+  im += (double)x.z * y.w - (double)x.w * y.z;
+}
+__device__ __forceinline__ void inner_add(double2 x, double2 y, double &re, double &im) {
+  re += x.x * y.x + x.y * y.y;
+  im += x.x * y.y - x.y * y.x;
 }
 
-// Sums `cols` interleaved columns of `rows` partial rows: out[c] = sum_r p[r*cols + c].
-__global__ void __launch_bounds__(kRedThreads) k_sum_columns(const double *__restrict__ p, int rows,
-                                                            int cols, double *__restrict__ out) {
-  for (int c = blockIdx.x; c < cols; c += gridDim.x) {
-    double acc = 0;
-    for (int r = threadIdx.x; r < rows; r += kRedThreads) acc += p[(size_t)r * cols + c];
-    acc = block_sum(acc);
-    if (threadIdx.x == 0) out[c] = acc;
-    __syncthreads();
+// out = <a|b> (re, im).  Bound by the two streams: four 16-byte loads of each in
+// flight a thread (one amplitude a time took 556 us for two 27-qubit complex64
+// states, 0.60 of the copy peak; now 356 us).
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads) k_inner(const T *__restrict__ a, const T *__restrict__ b,
+                                                      uint64_t n_vec, double *partial,
+                                                      double *__restrict__ out) {
+  using V = typename V16<T>::type;
+  const V *av = reinterpret_cast<const V *>(a);
+  const V *bv = reinterpret_cast<const V *>(b);
+  double re[4] = {}, im[4] = {};
+  const uint64_t stride = (uint64_t)gridDim.x * kRedThreads;
+  uint64_t i = (uint64_t)blockIdx.x * kRedThreads + threadIdx.x;
+  for (; i + 3 * stride < n_vec; i += 4 * stride) {
+    V x[4], y[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = av[i + u * stride];
+      y[u] = bv[i + u * stride];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) inner_add(x[u], y[u], re[u], im[u]);
   }
+  for (; i < n_vec; i += stride) inner_add(av[i], bv[i], re[0], im[0]);
+  if (n_vec == 0 && blockIdx.x == 0 && threadIdx.x == 0) {  // one complex64 amplitude: half a vector
+    re[0] = (double)a[0] * b[0] + (double)a[1] * b[1];
+    im[0] = (double)a[0] * b[1] - (double)a[1] * b[0];
+  }
+  const double r = block_sum((re[0] + re[1]) + (re[2] + re[3]));
+  __syncthreads();
+  const double m = block_sum((im[0] + im[1]) + (im[2] + im[3]));
+  if (threadIdx.x == 0) {
+    partial[2 * blockIdx.x] = r;
+    partial[2 * blockIdx.x + 1] = m;
+  }
+  if (last_block()) fold_columns(partial, (int)gridDim.x, 2, out);
 }
 
 constexpr int kMaxPopQubits = 40;
 
-// Per-qubit populations P(q = 1) and the total norm in one pass.  Each thread
-// walks 8-amplitude chunks: the chunk's high index bits are constant, so the
-// chunk sum is added once per high qubit; the 3 low bits are split per amp.
+// |a|^2 of the amplitudes of a 16-byte vector: two in FP32, one in FP64.
+__device__ __forceinline__ double prob_lo(float4 v) { return (double)v.x * v.x + (double)v.y * v.y; }
+__device__ __forceinline__ double prob_hi(float4 v) { return (double)v.z * v.z + (double)v.w * v.w; }
+__device__ __forceinline__ double prob_lo(double2 v) { return v.x * v.x + v.y * v.y; }
+__device__ __forceinline__ double prob_hi(double2) { return 0.0; }
+
+// The state as rows of kRedThreads 16-byte vectors: bits of an amplitude's index
+// are [row | thread | place in the vector].
+template <typename T> constexpr uint32_t vec_bits() { return sizeof(T) == 4 ? 1 : 0; }
+template <typename T> constexpr uint32_t row_bits() { return 8 + vec_bits<T>(); }
+constexpr uint32_t kPopRowBits = 3;  // rows a thread takes at once, all loads in flight
+
+// Per-qubit populations P(q = 1) and the total norm in one pass, for states of at
+// least one chunk of 8 rows.  A thread's place in a row is fixed, so its total
+// serves every qubit that indexes threads, at the end; the three lowest row bits
+// are split inside a chunk; the chunk's total is added once for every set bit of
+// the chunk's index.  That is about five FP64 operations an amplitude, which the
+// loads (128 bytes in flight a thread) cover.  27-qubit complex64: 498 -> 190
+// us (a thread took 8 consecutive amplitudes, 128 bytes apart from its
+// neighbour's).
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_populations(const T *__restrict__ x, uint32_t n,
-                                                            double *__restrict__ partial) {
+__global__ void __launch_bounds__(kRedThreads, 2) k_populations(const T *__restrict__ x, uint32_t n,
+                                                               double *partial, double *__restrict__ out) {
+  using V = typename V16<T>::type;
+  constexpr uint32_t VB = vec_bits<T>(), CB = row_bits<T>() + kPopRowBits;
+  constexpr int R = 1 << kPopRowBits;
+  const V *xv = reinterpret_cast<const V *>(x);
+  const uint64_t n_chunks = 1ull << (n - CB);
+  double odd = 0, row[kPopRowBits] = {}, tot = 0, high[kMaxPopQubits - CB] = {};
+  for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+    V v[R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) v[u] = xv[(c * R + u) * kRedThreads + threadIdx.x];
+    double s[R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      s[u] = prob_lo(v[u]);
+      if (VB) {
+        const double h = prob_hi(v[u]);
+        odd += h;
+        s[u] += h;
+      }
+    }
+    const double p01 = s[0] + s[1], p23 = s[2] + s[3], p45 = s[4] + s[5], p67 = s[6] + s[7];
+    row[0] += (s[1] + s[3]) + (s[5] + s[7]);
+    row[1] += p23 + p67;
+    const double top = p45 + p67, all = (p01 + p23) + top;
+    row[2] += top;
+    tot += all;
+#pragma unroll
+    for (uint32_t q = 0; q < kMaxPopQubits - CB; ++q)
+      if ((c >> q) & 1) high[q] += all;
+  }
+  // columns of this block's partial row: qubits 0 .. n - 1, then the norm
+  __shared__ double red[kRedThreads / 32];
+  double *mine = partial + (size_t)blockIdx.x * (n + 1);
+  auto put = [&](uint32_t column, double v) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0;
+      for (int w = 0; w < kRedThreads / 32; ++w) t += red[w];
+      mine[column] = t;
+    }
+    __syncthreads();
+  };
+  if (VB) put(0, odd);
+#pragma unroll
+  for (uint32_t b = 0; b < 8; ++b) put(VB + b, (threadIdx.x >> b) & 1 ? tot : 0.0);
+#pragma unroll
+  for (uint32_t b = 0; b < kPopRowBits; ++b) put(row_bits<T>() + b, row[b]);
+#pragma unroll
+  for (uint32_t q = 0; q < kMaxPopQubits - CB; ++q)
+    if (CB + q < n) put(CB + q, high[q]);
+  put(n, tot);
+  if (last_block()) fold_columns(partial, (int)gridDim.x, (int)n + 1, out);
+}
+
+// The same for a state below one chunk: one block, amplitude by amplitude.
+template <typename T>
+__global__ void __launch_bounds__(kRedThreads) k_populations_small(const T *__restrict__ x, uint32_t n,
+                                                                  double *__restrict__ out) {
   using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
   const V *xv = reinterpret_cast<const V *>(x);
-  const uint64_t n_amps = 1ull << n;
-  const uint32_t cb = n < 3 ? n : 3;  // chunk bits
-  const uint64_t n_chunks = n_amps >> cb;
-  double acc[kMaxPopQubits + 1];
-#pragma unroll
-  for (int q = 0; q <= kMaxPopQubits; ++q) acc[q] = 0;
-  const uint64_t stride = (uint64_t)gridDim.x * kRedThreads;
-  for (uint64_t c = (uint64_t)blockIdx.x * kRedThreads + threadIdx.x; c < n_chunks; c += stride) {
-    double lo[3] = {0, 0, 0}, tot = 0;
-    for (uint32_t j = 0; j < (1u << cb); ++j) {
-      const V v = xv[(c << cb) + j];
-      const double p = (double)v.x * v.x + (double)v.y * v.y;
-      tot += p;
-      if (j & 1) lo[0] += p;
-      if (j & 2) lo[1] += p;
-      if (j & 4) lo[2] += p;
-    }
-    acc[kMaxPopQubits] += tot;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) acc[q] += lo[q];
-#pragma unroll
-    for (int q = 3; q < kMaxPopQubits; ++q)
-      if ((uint32_t)q < n && ((c >> (q - 3)) & 1)) acc[q] += tot;
-  }
-  __shared__ double red[kRedThreads / 32];
-#pragma unroll
-  for (int q = 0; q <= kMaxPopQubits; ++q) {
-    if (q < (int)n || q == kMaxPopQubits) {
-      double v = warp_sum(acc[q]);
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double t = 0;
-        for (int w = 0; w < kRedThreads / 32; ++w) t += red[w];
-        partial[(size_t)blockIdx.x * (kMaxPopQubits + 1) + q] = t;
+  const int lane = threadIdx.x & 31;
+  // a warp a column
+  for (uint32_t c = threadIdx.x >> 5; c <= n; c += kRedThreads / 32) {
+    double acc = 0;
+    for (uint32_t i = lane; i < (1u << n); i += 32)
+      if (c == n || ((i >> c) & 1)) {
+        const V v = xv[i];
+        acc += (double)v.x * v.x + (double)v.y * v.y;
       }
-      __syncthreads();
-    }
+    acc = warp_sum(acc);
+    if (lane == 0) out[c] = acc;
   }
 }
 
-// Marginal probabilities over m measured qubits: per-block bins in shared
-// memory (FP64 shared atomics), written as per-block partial rows.
+// Marginal probabilities over m distinct measured qubits (ascending).  A block
+// takes rows of one value of the measured row bits (`high`), so a thread's bin
+// never changes while it sums: no atomics.  At the end lanes that differ only in
+// unmeasured lane bits are summed by shuffles, warps that differ only in
+// unmeasured warp bits through shared memory, and the block writes one partial
+// per value of the measured bits inside a row.  One FP64 shared atomic an
+// amplitude, as before, took 3.2 ms for 5 qubits of a 27-qubit complex64 state
+// and 13.4 ms for one high qubit; now 185 and 195 us.
+struct MarginalArgs {
+  uint64_t row_mask;   // measured bits of the row index
+  uint32_t thread_mask;  // measured bits of the thread index
+  uint32_t vec_measured;  // the place in the vector is measured
+  uint32_t n_rows_log2;
+  uint32_t segs_log2;  // blocks that share a value of the measured row bits
+  uint32_t high_bits, in_bits;  // popcounts: row_mask; thread_mask + vec
+};
+
+__device__ __forceinline__ uint64_t deposit(uint64_t v, uint64_t mask) {
+  uint64_t r = 0;
+  for (; mask; mask &= mask - 1, v >>= 1)
+    if (v & 1) r |= mask & (~mask + 1);
+  return r;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_marginal(const T *__restrict__ x, uint32_t n,
-                                                         const uint32_t *__restrict__ measured,
-                                                         uint32_t m, double *__restrict__ partial) {
-  using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
-  extern __shared__ double bins[];
-  const uint32_t nb = 1u << m;
-  for (uint32_t i = threadIdx.x; i < nb; i += kRedThreads) bins[i] = 0;
-  __shared__ uint32_t mq[16];
-  if (threadIdx.x < m) mq[threadIdx.x] = measured[threadIdx.x];
-  __syncthreads();
+__global__ void __launch_bounds__(kRedThreads) k_marginal_rows(const T *__restrict__ x, uint32_t n,
+                                                              const MarginalArgs a,
+                                                              double *__restrict__ partial) {
+  using V = typename V16<T>::type;
+  constexpr uint32_t VB = vec_bits<T>();
   const V *xv = reinterpret_cast<const V *>(x);
-  const uint64_t n_amps = 1ull << n;
-  const uint64_t stride = (uint64_t)gridDim.x * kRedThreads;
-  for (uint64_t i = (uint64_t)blockIdx.x * kRedThreads + threadIdx.x; i < n_amps; i += stride) {
-    const V v = xv[i];
-    uint32_t bin = 0;
-    for (uint32_t j = 0; j < m; ++j) bin |= (uint32_t)((i >> mq[j]) & 1) << j;
-    atomicAdd(&bins[bin], (double)v.x * v.x + (double)v.y * v.y);
+  const uint64_t high = blockIdx.x >> a.segs_log2, seg = blockIdx.x & ((1u << a.segs_log2) - 1);
+  const uint64_t free_mask = ((1ull << a.n_rows_log2) - 1) & ~a.row_mask;
+  const uint64_t per = 1ull << (a.n_rows_log2 - a.high_bits - a.segs_log2);  // rows of this block
+  // rows in ascending order of their unmeasured bits
+  uint64_t r = deposit(seg * per, free_mask);
+  const uint64_t fixed = deposit(high, a.row_mask);
+  double lo[2] = {}, hi[2] = {};
+  const bool live = ((uint64_t)threadIdx.x << VB) < (1ull << n);
+  if (live) {
+    uint64_t k = 0;
+    for (; k + 8 <= per; k += 8) {
+      V v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        v[u] = xv[(r | fixed) * kRedThreads + threadIdx.x];
+        r = ((r | ~free_mask) + 1) & free_mask;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        lo[u & 1] += prob_lo(v[u]);
+        if (VB) hi[u & 1] += prob_hi(v[u]);
+      }
+    }
+    for (; k < per; ++k) {
+      const V v = xv[(r | fixed) * kRedThreads + threadIdx.x];
+      r = ((r | ~free_mask) + 1) & free_mask;
+      lo[0] += prob_lo(v);
+      if (VB) hi[0] += prob_hi(v);
+    }
+  }
+  double p[2] = {lo[0] + lo[1], hi[0] + hi[1]};
+  if (!a.vec_measured) p[0] += p[1];
+  __shared__ double sm[2][kRedThreads];
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+      const double other = __shfl_xor_sync(0xffffffffu, p[v], 1 << b);
+      if (!((a.thread_mask >> b) & 1)) p[v] += other;
+    }
+    sm[v][threadIdx.x] = p[v];
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < nb; i += kRedThreads)
-    partial[(size_t)blockIdx.x * nb + i] = bins[i];
+  const uint32_t warp_free = 0xe0u & ~a.thread_mask;
+  for (uint32_t o = threadIdx.x; o < (1u << a.in_bits); o += kRedThreads) {
+    const uint32_t v = a.vec_measured ? o & 1 : 0;
+    const uint32_t t = (uint32_t)deposit(a.vec_measured ? o >> 1 : o, a.thread_mask);
+    double sum = 0;
+    uint32_t w = 0;
+    do {
+      sum += sm[v][t | w];
+      w = ((w | ~warp_free) + 1) & warp_free;
+    } while (w);
+    partial[((uint64_t)blockIdx.x << a.in_bits) + o] = sum;
+  }
+}
+
+// out[bin] = sum over the segments that share it (bins: measured row bits above
+// the measured bits inside a row).
+__global__ void __launch_bounds__(kRedThreads) k_marginal_fold(const double *__restrict__ partial,
+                                                              uint32_t bins, uint32_t in_bits,
+                                                              uint32_t segs_log2, double *__restrict__ out) {
+  for (uint32_t b = blockIdx.x * (kRedThreads / 32) + (threadIdx.x >> 5); b < bins;
+       b += gridDim.x * (kRedThreads / 32)) {
+    const uint32_t high = b >> in_bits, in = b & ((1u << in_bits) - 1);
+    double acc = 0;
+    for (uint32_t s = threadIdx.x & 31; s < (1u << segs_log2); s += 32)
+      acc += partial[((((uint64_t)high << segs_log2) + s) << in_bits) + in];
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) out[b] = acc;
+  }
 }
 
 // A table of powers indexed by a popcount (0 .. kMaxPopQubits), passed to the
@@ -288,7 +475,7 @@ struct PopcTable {
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_damp_sums(const T *__restrict__ x, uint32_t n,
                                                           uint64_t mask, const PopcTable tab,
-                                                          double *__restrict__ partial) {
+                                                          double *partial, double *__restrict__ out) {
   using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
   const V *xv = reinterpret_cast<const V *>(x);
   const uint64_t n_amps = 1ull << n;
@@ -307,6 +494,7 @@ __global__ void __launch_bounds__(kRedThreads) k_damp_sums(const T *__restrict__
     partial[2 * blockIdx.x] = t;
     partial[2 * blockIdx.x + 1] = d;
   }
+  if (last_block()) fold_columns(partial, (int)gridDim.x, 2, out);
 }
 
 // x_i *= scale * s^popc(i & mask): the no-jump branch of amplitude damping on
@@ -340,21 +528,15 @@ template <typename T>
 bool inner_impl(const void *a, const void *b, uint32_t n, double *re, double *im, cudaStream_t s,
                 std::string &err) {
   std::lock_guard<std::mutex> lock(g_scratch_mu);
-  const uint64_t amps = 1ull << n;
-  const unsigned grid = red_grid(amps);
-  double *const g_scratch = ensure_scratch(2 * (int)grid + 2, err);
-  if (!g_scratch) return false;
-  k_inner_pass1<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(a), static_cast<const T *>(b),
-                                                 amps, g_scratch);
-  k_sum_columns<<<2, kRedThreads, 0, s>>>(g_scratch, (int)grid, 2, g_scratch + 2 * grid);
-  double host[2];
-  if (!cuda_ok(cudaGetLastError(), "inner product launch", err) ||
-      !cuda_ok(cudaMemcpyAsync(host, g_scratch + 2 * grid, 16, cudaMemcpyDeviceToHost, s),
-               "cudaMemcpyAsync (inner product)", err) ||
-      !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (inner product)", err))
-    return false;
-  *re = host[0];
-  *im = host[1];
+  const uint64_t vec = (1ull << n) >> vec_bits<T>();
+  const unsigned grid = red_grid(vec);
+  Scratch *const sc = ensure_scratch(2 * (int)grid, err);
+  if (!sc) return false;
+  k_inner<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(a), static_cast<const T *>(b), vec,
+                                          sc->partial, sc->result);
+  if (!fetch_result(s, "inner product", err)) return false;
+  *re = sc->result[0];
+  *im = sc->result[1];
   return true;
 }
 
@@ -362,48 +544,68 @@ template <typename T>
 bool pop_impl(const void *x, uint32_t n, double *p1, double *norm, cudaStream_t s,
               std::string &err) {
   std::lock_guard<std::mutex> lock(g_scratch_mu);
-  const uint64_t chunks = (1ull << n) >> (n < 3 ? n : 3);
-  const unsigned grid = std::min<unsigned>(red_grid(chunks), 2 * sm_count());
-  constexpr int W = kMaxPopQubits + 1;
-  double *const g_scratch = ensure_scratch(W * ((int)grid + 1), err);
-  if (!g_scratch) return false;
-  cudaMemsetAsync(g_scratch, 0, sizeof(double) * W * grid, s);
-  k_populations<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, g_scratch);
-  k_sum_columns<<<W, kRedThreads, 0, s>>>(g_scratch, (int)grid, W, g_scratch + (size_t)W * grid);
-  std::vector<double> host(W);
-  if (!cuda_ok(cudaGetLastError(), "populations launch", err) ||
-      !cuda_ok(cudaMemcpyAsync(host.data(), g_scratch + (size_t)W * grid, sizeof(double) * W,
-                               cudaMemcpyDeviceToHost, s),
-               "cudaMemcpyAsync (populations)", err) ||
-      !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (populations)", err))
-    return false;
-  for (uint32_t q = 0; q < n; ++q) p1[q] = host[q];
-  if (norm) *norm = host[kMaxPopQubits];
+  constexpr uint32_t CB = row_bits<T>() + kPopRowBits;
+  const uint64_t chunks = n >= CB ? 1ull << (n - CB) : 1;
+  const unsigned grid = (unsigned)std::min<uint64_t>(chunks, 2ull * sm_count());
+  Scratch *const sc = ensure_scratch((int)((n + 1) * grid), err);
+  if (!sc) return false;
+  if (n >= CB)
+    k_populations<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->partial, sc->result);
+  else
+    k_populations_small<T><<<1, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->result);
+  if (!fetch_result(s, "populations", err)) return false;
+  for (uint32_t q = 0; q < n; ++q) p1[q] = sc->result[q];
+  if (norm) *norm = sc->result[n];
   return true;
 }
 
 template <typename T>
 bool marg_impl(const void *x, uint32_t n, const uint32_t *measured, uint32_t m, double *out,
                cudaStream_t s, std::string &err) {
+  // the distinct measured qubits, ascending; the caller's order (and any qubit
+  // listed twice) is restored from their bins at the end
+  uint64_t mask = 0;
+  for (uint32_t j = 0; j < m; ++j) mask |= 1ull << measured[j];
+  constexpr uint32_t VB = vec_bits<T>(), RB = row_bits<T>();
+  MarginalArgs a{};
+  a.vec_measured = VB ? (uint32_t)(mask & 1) : 0;
+  a.thread_mask = (uint32_t)((mask >> VB) & (kRedThreads - 1));
+  a.row_mask = mask >> RB;
+  a.n_rows_log2 = n > RB ? n - RB : 0;
+  a.high_bits = (uint32_t)__builtin_popcountll(a.row_mask);
+  a.in_bits = (uint32_t)__builtin_popcountll(mask) - a.high_bits;
+  // about 8 blocks an SM, each with at least 8 rows where there are that many
+  const uint32_t free_rows = a.n_rows_log2 - a.high_bits;
+  uint32_t want = 0;
+  while ((1u << (a.high_bits + want)) < 8u * (uint32_t)sm_count()) ++want;
+  a.segs_log2 = std::min(want, free_rows > 3 ? free_rows - 3 : 0);
+  const uint32_t bins = 1u << (a.high_bits + a.in_bits);
+  const unsigned grid = 1u << (a.high_bits + a.segs_log2);
   std::lock_guard<std::mutex> lock(g_scratch_mu);
-  const uint32_t nb = 1u << m;
-  const unsigned grid = std::min<unsigned>(red_grid(1ull << n), 2 * sm_count());
-  const int need = (int)(nb * (grid + 1)) + 16;
-  double *const g_scratch = ensure_scratch(need, err);
-  if (!g_scratch) return false;
-  uint32_t *dq = reinterpret_cast<uint32_t *>(g_scratch + (size_t)nb * (grid + 1));
-  if (!cuda_ok(cudaMemcpyAsync(dq, measured, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, s),
-               "cudaMemcpyAsync (measured qubits)", err))
-    return false;
-  k_marginal<T><<<grid, kRedThreads, sizeof(double) * nb, s>>>(static_cast<const T *>(x), n, dq, m,
-                                                              g_scratch);
-  k_sum_columns<<<std::min<uint32_t>(nb, 1024), kRedThreads, 0, s>>>(g_scratch, (int)grid, (int)nb,
-                                                                      g_scratch + (size_t)nb * grid);
-  return cuda_ok(cudaGetLastError(), "marginal launch", err) &&
-         cuda_ok(cudaMemcpyAsync(out, g_scratch + (size_t)nb * grid, sizeof(double) * nb,
-                                 cudaMemcpyDeviceToHost, s),
-                 "cudaMemcpyAsync (marginal)", err) &&
-         cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (marginal)", err);
+  Scratch *const sc = ensure_scratch((int)(grid << a.in_bits), err);
+  if (!sc) return false;
+  k_marginal_rows<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, a, sc->partial);
+  k_marginal_fold<<<std::min<uint32_t>((bins + 7) / 8, 512), kRedThreads, 0, s>>>(
+      sc->partial, bins, a.in_bits, a.segs_log2, sc->result);
+  if (!fetch_result(s, "marginal", err)) return false;
+  // out[i]: the bin whose bits are i's at the measured qubits' places
+  uint32_t bin[1u << 12], place[12];
+  bool listed_once = true;
+  for (uint32_t j = 0; j < m; ++j) {
+    place[j] = (uint32_t)__builtin_popcountll(mask & ((1ull << measured[j]) - 1));
+    for (uint32_t l = 0; l < j; ++l) listed_once = listed_once && measured[l] != measured[j];
+  }
+  bin[0] = 0;
+  out[0] = sc->result[0];
+  for (uint32_t i = 1; i < (1u << m); ++i) {
+    bin[i] = bin[i & (i - 1)] | 1u << place[__builtin_ctz(i)];
+    out[i] = sc->result[bin[i]];
+  }
+  if (!listed_once)  // bits of one qubit that disagree never occur
+    for (uint32_t i = 0; i < (1u << m); ++i)
+      for (uint32_t j = 0; j < m; ++j)
+        if (((i >> j) & 1) != ((bin[i] >> place[j]) & 1)) out[i] = 0.0;
+  return true;
 }
 
 PopcTable powers(double base, double first) {
@@ -421,19 +623,13 @@ bool damp_sums_impl(const void *x, uint32_t n, uint64_t mask, double gamma, doub
                     cudaStream_t s, std::string &err) {
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   const unsigned grid = red_grid(1ull << n);
-  double *const g_scratch = ensure_scratch(2 * (int)grid + 2, err);
-  if (!g_scratch) return false;
-  double res[2];
-  k_damp_sums<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, mask,
-                                               powers(1.0 - gamma, 1.0), g_scratch);
-  k_sum_columns<<<2, kRedThreads, 0, s>>>(g_scratch, (int)grid, 2, g_scratch + 2 * grid);
-  if (!cuda_ok(cudaGetLastError(), "damping sums launch", err) ||
-      !cuda_ok(cudaMemcpyAsync(res, g_scratch + 2 * grid, 16, cudaMemcpyDeviceToHost, s),
-               "cudaMemcpyAsync (damping sums)", err) ||
-      !cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (damping sums)", err))
-    return false;
-  *tot = res[0];
-  *wsum = res[1];
+  Scratch *const sc = ensure_scratch(2 * (int)grid, err);
+  if (!sc) return false;
+  k_damp_sums<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, mask, powers(1.0 - gamma, 1.0),
+                                              sc->partial, sc->result);
+  if (!fetch_result(s, "damping sums", err)) return false;
+  *tot = sc->result[0];
+  *wsum = sc->result[1];
   return true;
 }
 

@@ -53,6 +53,7 @@ namespace {
 
 constexpr int kSmpThreads = 256;
 constexpr uint32_t kMaxChunkBits = 12;  // 4096 amplitudes, 16 a thread in the prefix pass
+constexpr uint32_t kFullPer = (1u << kMaxChunkBits) / kSmpThreads;  // a thread's amplitudes of a full chunk
 constexpr int kScanThreads = 1024;
 constexpr uint32_t kScanPer = 8;  // elements a scan thread sums in order
 constexpr uint32_t kMaxMeasured = 64;
@@ -118,10 +119,22 @@ __global__ void __launch_bounds__(kSmpThreads) k_chunk_totals(const T *__restric
   const V *xv = reinterpret_cast<const V *>(x) + (chunk << cb);
   uint64_t q = 0;
   double p = 0.0;
-  for (uint32_t i = threadIdx.x; i < (1u << cb); i += kSmpThreads) {
-    const double pi = prob(xv[i]);
-    q += fix(pi, scale);
-    p += pi;
+  if (cb == kMaxChunkBits) {  // a full chunk: every load of the thread in flight at once
+    V v[kFullPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kFullPer; ++u) v[u] = xv[threadIdx.x + u * kSmpThreads];
+#pragma unroll
+    for (uint32_t u = 0; u < kFullPer; ++u) {
+      const double pi = prob(v[u]);
+      q += fix(pi, scale);
+      p += pi;
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < (1u << cb); i += kSmpThreads) {
+      const double pi = prob(xv[i]);
+      q += fix(pi, scale);
+      p += pi;
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -306,7 +319,18 @@ __global__ void __launch_bounds__(kSmpThreads) k_sample_assign(
   const uint32_t nt = c < (uint32_t)kSmpThreads ? c : (uint32_t)kSmpThreads;
   const uint32_t per = c / nt;
   const V *xv = reinterpret_cast<const V *>(x) + (chunk << cb);
-  for (uint32_t i = threadIdx.x; i < c; i += kSmpThreads) q[i + (i >> 4)] = fix(prob(xv[i]), scale);
+  if (cb == kMaxChunkBits) {
+    V v[kFullPer];
+#pragma unroll
+    for (uint32_t u = 0; u < kFullPer; ++u) v[u] = xv[threadIdx.x + u * kSmpThreads];
+#pragma unroll
+    for (uint32_t u = 0; u < kFullPer; ++u) {
+      const uint32_t i = threadIdx.x + u * kSmpThreads;
+      q[i + (i >> 4)] = fix(prob(v[u]), scale);
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < c; i += kSmpThreads) q[i + (i >> 4)] = fix(prob(xv[i]), scale);
+  }
   __syncthreads();
   uint64_t s = 0;
   if (threadIdx.x < nt)
