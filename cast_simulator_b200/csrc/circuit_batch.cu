@@ -8,25 +8,30 @@
 // independent circuits - different qubit counts, depths and precisions - runs
 // in ONE launch:
 //
-//  * a persistent grid of CTAs (512 threads); each CTA claims the next circuit
-//    from a device work counter, so long and short circuits balance (the host
-//    orders the batch longest first);
-//  * the CTA owns the circuit's statevector (the caller's device buffer, at
-//    most 2^20 amplitudes: 16 MiB in complex128) and runs every fused gate
-//    (k <= 4) on it in place, one thread per gather group, a __syncthreads()
-//    between gates; the gate matrix is staged in shared memory first.  Small
-//    states stay in L1/L2 across the whole circuit;
-//  * optionally it starts from |0...0> (written by the CTA itself);
-//  * at the end it reduces, in FP64 and in a fixed order, the norm and
+//  * a persistent grid of CTAs; each CTA claims the next circuit from a device
+//    work counter, so long and short circuits balance (the host orders the batch
+//    longest first);
+//  * a circuit whose state fits (complex128 7..13 qubits, complex64 3..14) lives in
+//    shared memory from its first gate to its last: every fused gate (k <= 4) is
+//    applied there with the tile code of the merged passes (gate_tile.cuh), the
+//    next gate's matrix and walk copied in behind it, and the state is written to
+//    the caller's buffer once.  Gate after gate through L1 and L2, as the larger
+//    circuits still run, a gate waits for its loads and for a matrix entry from
+//    shared memory for every four FMAs: 256 circuits of 8..13 qubits took 700 us,
+//    now 238 (kernel 246 -> 140);
+//  * the others run every gate in place on the caller's device buffer (at most 2^20
+//    amplitudes: 16 MiB in complex128), one thread per gather group;
+//  * optionally a circuit starts from |0...0> (written by the CTA itself);
+//  * at the end the CTA reduces, in FP64 and in a fixed order, the norm and
 //    P(q = 1) of every qubit, and writes <Z_q> = (norm - 2 P(q = 1)) / norm.
 //
 // Matrices are snapped with the plain path's zero / +-1 rule
 // (src/cpp/cuda/cuda_gen.cpp:84-103) and stored in the circuit's precision.
-// Everything a batch needs - circuit table, op list, matrices, the work
-// counter - is packed into one pinned host buffer and sent with one copy; the
-// <Z> table comes back with one copy: three operations on one stream a batch.
+// The circuit table, op list and matrices go to the device at the first run after
+// a change of the batch; a run resets the work counter, launches, and copies the
+// <Z> table back: three operations on one stream.
 #include "../../include/cast_b200.h"
-#include "internal.hpp"
+#include "gate_tile.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -35,13 +40,17 @@
 #include <numeric>
 #include <vector>
 
+#include <cuda_pipeline.h>
+
 namespace {
 
 using cb2::cuda_ok;
 using cb2::write_err;
 using cb2::clear_err;
 
-constexpr int kBThreads = 512;
+// Threads a CTA: 256 when every circuit of a batch is resident (two CTAs an SM for
+// small states), 512 when one streams its state from memory (loads in flight).
+constexpr int kBResidentThreads = 256, kBThreads = 512;
 constexpr uint32_t kBatchMaxQubits = 20;
 constexpr uint32_t kBatchMaxGate = 4;
 constexpr uint32_t kBatchMagic = 0xB47C4001u;
@@ -54,13 +63,31 @@ struct BCircuit {
   uint32_t n_ops;
   uint32_t init_zero;
   uint32_t z_off;   // first <Z> slot of this circuit
+  uint32_t resident;  // the state is held in shared memory
+  uint32_t pad;
 };
 
-struct BOp {
-  uint32_t k;
-  uint32_t q[kBatchMaxGate];
+struct alignas(16) BOp {
   uint32_t mat;  // byte offset of the matrix in the pool (16-byte aligned)
+  uint32_t mat_bytes;
+  uint32_t k;    // of the gate, or of its laid-out form (3 or 4) when resident
+  uint32_t q[kBatchMaxGate];
+  union {  // resident circuits: the walk of the tile
+    cb2::PassGateArgs a64;
+    cb2::PassGateArgs32 a32;
+  };
 };
+
+// Shared memory: two gates' matrices (the resident form's 4-qubit matrix in
+// complex128 is the largest) and their ops, then a resident circuit's state.
+constexpr uint32_t kBMatBytes = 2 * 256 * sizeof(double);
+constexpr uint32_t kBStateOffset = 2 * kBMatBytes + 2 * ((sizeof(BOp) + 15) & ~15u);
+
+// Sizes whose state is held in shared memory: at least the tile code's smallest
+// tile, at most 128 KB.
+bool resident_size(uint32_t n, uint32_t prec) {
+  return prec ? n >= cb2::kTileMin64 && n <= cb2::kTileMax64 : n >= 3 && n <= cb2::kTileMax32;
+}
 
 struct BHeader {
   uint32_t next;  // work counter (zero in every upload)
@@ -81,8 +108,8 @@ template <typename V> __device__ __forceinline__ V cmac(V m, V x, V acc) {
   return acc;
 }
 
-// One fused k-qubit gate applied in place: thread t takes groups t, t + 512, ...
-template <typename T, int K>
+// One fused k-qubit gate applied in place: thread t takes groups t, t + NT, ...
+template <int NT, typename T, int K>
 __device__ __noinline__ void batch_gate(typename C2<T>::type *sv, uint32_t n, const uint32_t *q,
                                         const typename C2<T>::type *M) {
   using V = typename C2<T>::type;
@@ -91,7 +118,7 @@ __device__ __noinline__ void batch_gate(typename C2<T>::type *sv, uint32_t n, co
 #pragma unroll
   for (int b = 0; b < K; ++b) lo[b] = (1u << q[b]) - 1;
   const uint32_t ng = 1u << (n - K);
-  for (uint32_t g = threadIdx.x; g < ng; g += kBThreads) {
+  for (uint32_t g = threadIdx.x; g < ng; g += NT) {
     uint32_t base = g;
 #pragma unroll
     for (int b = 0; b < K; ++b) base = ((base & ~lo[b]) << 1) | (base & lo[b]);
@@ -121,21 +148,65 @@ __device__ __noinline__ void batch_gate(typename C2<T>::type *sv, uint32_t n, co
 }
 
 struct BShared {
-  double2 mat[1u << (2 * kBatchMaxGate)];  // 4 KiB: the largest matrix in complex128
-  double red[kBThreads / 32][kBatchMaxQubits + 1];
+  double red[kBThreads / 32][6 + kBatchMaxQubits];
   BCircuit circ;
   uint32_t claim;
 };
 
-template <typename T>
-__device__ void run_circuit(BShared &S, const BOp *__restrict__ ops, const char *__restrict__ pool,
-                            double *__restrict__ out_z) {
+// <Z_q> of a state of 2^n amplitudes with probabilities prob(i), i = u RT + thread,
+// by the first RT threads of the CTA (a resident circuit gives the same bits
+// whatever the CTA's size).  A thread's low index bits are fixed, so its total
+// serves their qubits.
+template <int RT, typename P>
+__device__ __forceinline__ void reduce_z(BShared &S, uint32_t n, P prob, double *__restrict__ out_z) {
+  constexpr uint32_t TB = RT == 512 ? 9 : 8;
+  static_assert(RT == 1 << TB, "a power of two of threads");
+  constexpr uint32_t HIGH = kBatchMaxQubits - TB;
+  double tot = 0.0, high[HIGH];
+#pragma unroll
+  for (uint32_t q = 0; q < HIGH; ++q) high[q] = 0.0;
+  for (uint32_t u = 0; threadIdx.x < RT && (u << TB) + threadIdx.x < (1u << n); ++u) {
+    const double p = prob((u << TB) + threadIdx.x);
+    tot += p;
+#pragma unroll
+    for (uint32_t q = 0; q < HIGH; ++q)
+      if ((u >> q) & 1) high[q] += p;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto put = [&](uint32_t slot, double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) S.red[warp][slot] = v;
+  };
+#pragma unroll
+  for (uint32_t b = 0; b < 5; ++b) put(b, (lane >> b) & 1 ? tot : 0.0);
+  put(5, tot);
+#pragma unroll
+  for (uint32_t q = 0; q < HIGH; ++q)
+    if (TB + q < n) put(6 + q, high[q]);
+  __syncthreads();
+  if (threadIdx.x < n) {
+    const uint32_t q = threadIdx.x;
+    double all = 0.0, p1 = 0.0;
+    for (uint32_t w = 0; w < RT / 32; ++w) {
+      all += S.red[w][5];
+      p1 += q < 5 ? S.red[w][q] : q < TB ? ((w >> (q - 5)) & 1 ? S.red[w][5] : 0.0) : S.red[w][6 + q - TB];
+    }
+    out_z[q] = all > 0.0 ? (all - 2.0 * p1) / all : 0.0;
+  }
+  __syncthreads();
+}
+
+// A circuit whose state stays in device memory.
+template <int NT, typename T>
+__device__ void run_streamed(BShared &S, unsigned char *smem, const BOp *__restrict__ ops,
+                             const char *__restrict__ pool, double *__restrict__ out_z) {
   using V = typename C2<T>::type;
   const BCircuit c = S.circ;
   V *sv = reinterpret_cast<V *>(c.sv);
   const uint32_t N = 1u << c.n;
   if (c.init_zero) {
-    for (uint32_t i = threadIdx.x; i < N; i += kBThreads) {
+    for (uint32_t i = threadIdx.x; i < N; i += NT) {
       V v;
       v.x = i == 0 ? (T)1 : (T)0;
       v.y = 0;
@@ -143,58 +214,92 @@ __device__ void run_circuit(BShared &S, const BOp *__restrict__ ops, const char 
     }
     __syncthreads();
   }
-  V *Msm = reinterpret_cast<V *>(S.mat);
+  V *Msm = reinterpret_cast<V *>(smem);
   for (uint32_t oi = 0; oi < c.n_ops; ++oi) {
-    const BOp op = ops[c.op_begin + oi];
+    const BOp &op = ops[c.op_begin + oi];
     const V *Mg = reinterpret_cast<const V *>(pool + op.mat);
-    const uint32_t entries = 1u << (2 * op.k);
-    for (uint32_t i = threadIdx.x; i < entries; i += kBThreads) Msm[i] = Mg[i];
+    const uint32_t k = op.k, entries = 1u << (2 * k);
+    for (uint32_t i = threadIdx.x; i < entries; i += NT) Msm[i] = Mg[i];
     __syncthreads();
-    switch (op.k) {
-    case 1: batch_gate<T, 1>(sv, c.n, op.q, Msm); break;
-    case 2: batch_gate<T, 2>(sv, c.n, op.q, Msm); break;
-    case 3: batch_gate<T, 3>(sv, c.n, op.q, Msm); break;
-    default: batch_gate<T, 4>(sv, c.n, op.q, Msm); break;
+    switch (k) {
+    case 1: batch_gate<NT, T, 1>(sv, c.n, op.q, Msm); break;
+    case 2: batch_gate<NT, T, 2>(sv, c.n, op.q, Msm); break;
+    case 3: batch_gate<NT, T, 3>(sv, c.n, op.q, Msm); break;
+    default: batch_gate<NT, T, 4>(sv, c.n, op.q, Msm); break;
     }
     __syncthreads();
   }
-  // FP64 norm and P(q = 1) per qubit, reduced in a fixed order
-  double acc[kBatchMaxQubits + 1];
-#pragma unroll
-  for (uint32_t q = 0; q <= kBatchMaxQubits; ++q) acc[q] = 0.0;
-  for (uint32_t i = threadIdx.x; i < N; i += kBThreads) {
+  reduce_z<NT>(S, c.n, [&](uint32_t i) {
     const V v = sv[i];
-    const double p = (double)v.x * v.x + (double)v.y * v.y;
-    acc[kBatchMaxQubits] += p;
-#pragma unroll
-    for (uint32_t q = 0; q < kBatchMaxQubits; ++q)
-      if ((i >> q) & 1) acc[q] += p;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (uint32_t q = 0; q <= kBatchMaxQubits; ++q) {
-    double v = acc[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) S.red[warp][q] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < c.n) {
-    double tot = 0.0, p1 = 0.0;
-    for (int w = 0; w < kBThreads / 32; ++w) {
-      tot += S.red[w][kBatchMaxQubits];
-      p1 += S.red[w][threadIdx.x];
-    }
-    out_z[c.z_off + threadIdx.x] = tot > 0.0 ? (tot - 2.0 * p1) / tot : 0.0;
-  }
-  __syncthreads();
+    return (double)v.x * v.x + (double)v.y * v.y;
+  }, out_z + c.z_off);
 }
 
-__global__ void __launch_bounds__(kBThreads, 1)
+// A circuit whose state is held in shared memory.
+template <int NT, typename T>
+__device__ void run_resident(BShared &S, unsigned char *smem, const BOp *__restrict__ ops,
+                             const char *__restrict__ pool, double *__restrict__ out_z) {
+  using V = typename C2<T>::type;
+  constexpr bool F64 = sizeof(T) == 8;
+  const BCircuit c = S.circ;
+  V *sv = reinterpret_cast<V *>(c.sv);
+  V *s = reinterpret_cast<V *>(smem + kBStateOffset);
+  BOp *const slots = reinterpret_cast<BOp *>(smem + 2 * kBMatBytes);
+  auto place = [](uint32_t i) { return F64 ? cb2::pass_swz(i) : cb2::pass_swz32(i); };
+  const uint32_t N = 1u << c.n;
+  for (uint32_t i = threadIdx.x; i < N; i += NT) {
+    V v;
+    v.x = i == 0 ? (T)1 : (T)0;
+    v.y = 0;
+    s[place(i)] = c.init_zero ? v : sv[i];
+  }
+  const BOp *const op = ops + c.op_begin;
+  // the copies of gate i's matrix and walk, given where its matrix is
+  auto fetch = [&](uint32_t i, uint2 where) {
+    unsigned char *to = smem + (i & 1) * kBMatBytes;
+    for (uint32_t b = 16 * threadIdx.x; b < where.y; b += 16 * NT)
+      __pipeline_memcpy_async(to + b, pool + where.x + b, 16);
+    if (threadIdx.x < sizeof(BOp) / 16)
+      __pipeline_memcpy_async(reinterpret_cast<char *>(&slots[i & 1]) + 16 * threadIdx.x,
+                              reinterpret_cast<const char *>(op + i) + 16 * threadIdx.x, 16);
+  };
+  auto where = [&](uint32_t i) { return *reinterpret_cast<const uint2 *>(op + i); };
+  if (c.n_ops) fetch(0, where(0));
+  uint2 next = c.n_ops > 1 ? where(1) : make_uint2(0, 0);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (uint32_t oi = 0; oi < c.n_ops; ++oi) {
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    __syncthreads();  // the gate before is done; this one's matrix and walk are here
+    if (oi + 1 < c.n_ops) fetch(oi + 1, next);
+    if (oi + 2 < c.n_ops) next = where(oi + 2);
+    const unsigned char *mat = smem + (oi & 1) * kBMatBytes;
+    const BOp &o = slots[oi & 1];
+    if constexpr (F64) {
+      const double *m = reinterpret_cast<const double *>(mat);
+      if (o.k == 4) cb2::pass_gate4_full<NT / 32>(s, m, o.a64, N >> 7, warp, lane);
+      else cb2::pass_gate3<NT / 32>(s, m, o.a64, N >> 6, warp, lane);
+    } else {
+      const float *m = reinterpret_cast<const float *>(mat);
+      if (o.k == 4) cb2::pass_gate32<NT, 4, 2, 2, false>(s, m, o.a32, c.n);
+      else cb2::pass_gate32<NT, 3, 1, 2, false>(s, m, o.a32, c.n);
+    }
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < N; i += NT) sv[i] = s[place(i)];
+  reduce_z<kBResidentThreads>(S, c.n, [&](uint32_t i) {
+    const V v = s[place(i)];
+    return (double)v.x * v.x + (double)v.y * v.y;
+  }, out_z + c.z_off);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == kBResidentThreads ? 2 : 1)
     k_circuit_batch(BHeader *__restrict__ hdr, const BCircuit *__restrict__ circs,
                     const BOp *__restrict__ ops, const char *__restrict__ pool,
                     double *__restrict__ out_z) {
   __shared__ BShared S;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const uint32_t n_circ = hdr->n_circuits;
   while (true) {
     if (threadIdx.x == 0) {
@@ -203,8 +308,13 @@ __global__ void __launch_bounds__(kBThreads, 1)
     }
     __syncthreads();
     if (S.claim >= n_circ) return;
-    if (S.circ.prec == 1) run_circuit<double>(S, ops, pool, out_z);
-    else run_circuit<float>(S, ops, pool, out_z);
+    if (S.circ.resident) {
+      if (S.circ.prec == 1) run_resident<NT, double>(S, smem_raw, ops, pool, out_z);
+      else run_resident<NT, float>(S, smem_raw, ops, pool, out_z);
+    } else {
+      if (S.circ.prec == 1) run_streamed<NT, double>(S, smem_raw, ops, pool, out_z);
+      else run_streamed<NT, float>(S, smem_raw, ops, pool, out_z);
+    }
   }
 }
 
@@ -218,18 +328,16 @@ struct Batch {
   std::vector<char> pool;   // matrices, each 16-byte aligned
   std::vector<uint64_t> cost;  // work estimate per circuit (ordering)
   uint32_t n_z = 0;
+  bool uploaded = false;  // the device buffer holds the circuits as they are now
   // device and pinned buffers, grown on demand and reused across runs
   char *dev = nullptr;
   size_t dev_cap = 0;
-  char *host = nullptr;
-  size_t host_cap = 0;
   double *host_z = nullptr;
   size_t host_z_cap = 0;
   int device = -1;
 
   ~Batch() {
     if (dev) cudaFree(dev);
-    if (host) cudaFreeHost(host);
     if (host_z) cudaFreeHost(host_z);
   }
 };
@@ -265,6 +373,11 @@ bool add_circuit(Batch &b, uint64_t sv, uint32_t n, uint8_t prec, uint32_t n_gat
   c.n_ops = n_gates;
   c.init_zero = init_zero ? 1 : 0;
   c.z_off = b.n_z;
+  c.resident = resident_size(n, prec) ? 1 : 0;
+  std::vector<uint32_t> tile_qubits(n);
+  std::iota(tile_qubits.begin(), tile_qubits.end(), 0u);
+  std::vector<double> frag64;
+  std::vector<float> frag32;
   std::vector<BOp> new_ops;
   std::vector<char> new_pool;
   size_t qoff = 0, moff = 0;
@@ -293,12 +406,24 @@ bool add_circuit(Batch &b, uint64_t sv, uint32_t n, uint8_t prec, uint32_t n_gat
     const size_t entries = 1ull << (2 * k);
     cb2::snap_matrix(g, mats + 2 * moff, ztol, otol);
     moff += entries;
-    const size_t bytes = entries * (prec ? 16 : 8);
+    size_t bytes = entries * (prec ? 16 : 8);
+    const void *from = prec ? (const void *)g.m64.data() : (const void *)g.m32.data();
+    if (c.resident) {
+      for (uint32_t j = 0; j < k; ++j) g.qubits[j] = op.q[j];
+      const cb2::PlacedGate placed = cb2::place_gate(g, tile_qubits);
+      op.k = placed.k;
+      frag64.clear();
+      frag32.clear();
+      if (prec) cb2::pack_gate(placed, n, false, frag64, op.a64);
+      else cb2::pack_gate32(placed, n, false, frag32, op.a32);
+      bytes = prec ? frag64.size() * sizeof(double) : frag32.size() * sizeof(float);
+      from = prec ? (const void *)frag64.data() : (const void *)frag32.data();
+    }
     op.mat = (uint32_t)(b.pool.size() + new_pool.size());
+    op.mat_bytes = (uint32_t)bytes;
     const size_t at = new_pool.size();
     new_pool.resize(align16(at + bytes));
-    if (prec) std::memcpy(new_pool.data() + at, g.m64.data(), bytes);
-    else std::memcpy(new_pool.data() + at, g.m32.data(), bytes);
+    std::memcpy(new_pool.data() + at, from, bytes);
     new_ops.push_back(op);
     cost += (uint64_t)entries << (n - k);  // complex multiply-adds of the pass
   }
@@ -308,11 +433,14 @@ bool add_circuit(Batch &b, uint64_t sv, uint32_t n, uint8_t prec, uint32_t n_gat
   }
   b.ops.insert(b.ops.end(), new_ops.begin(), new_ops.end());
   b.pool.insert(b.pool.end(), new_pool.begin(), new_pool.end());
+  b.uploaded = false;
   b.circs.push_back(c);
   b.cost.push_back(cost + (2ull << n));
   b.n_z += n;
   return true;
 }
+
+size_t smem_most() { return kBStateOffset + (sizeof(double2) << cb2::kTileMax64); }
 
 bool run_batch(Batch &b, double *out_z, cudaStream_t s, std::string &err) {
   const uint32_t nc = (uint32_t)b.circs.size();
@@ -324,36 +452,23 @@ bool run_batch(Batch &b, double *out_z, cudaStream_t s, std::string &err) {
     b.dev = nullptr;
     b.dev_cap = 0;
     b.device = dev;
+    b.uploaded = false;
   }
-  // longest first: the work counter hands them out in this order
-  std::vector<uint32_t> order(nc);
-  std::iota(order.begin(), order.end(), 0u);
-  std::stable_sort(order.begin(), order.end(),
-                   [&](uint32_t a, uint32_t c) { return b.cost[a] > b.cost[c]; });
   const size_t off_c = align16(sizeof(BHeader));
   const size_t off_o = align16(off_c + sizeof(BCircuit) * nc);
   const size_t off_p = align16(off_o + sizeof(BOp) * b.ops.size());
   const size_t off_z = align16(off_p + b.pool.size());
-  const size_t up = off_z, total = off_z + sizeof(double) * b.n_z;
+  const size_t total = off_z + sizeof(double) * b.n_z;
   if (b.dev_cap < total) {
     if (b.dev) cudaFree(b.dev);
     b.dev = nullptr;
+    b.uploaded = false;
     const size_t cap = std::max(total, b.dev_cap * 2);
     if (!cuda_ok(cudaMalloc(&b.dev, cap), "cudaMalloc (circuit batch)", err)) {
       b.dev_cap = 0;
       return false;
     }
     b.dev_cap = cap;
-  }
-  if (b.host_cap < up) {
-    if (b.host) cudaFreeHost(b.host);
-    b.host = nullptr;
-    const size_t cap = std::max(up, b.host_cap * 2);
-    if (!cuda_ok(cudaMallocHost(&b.host, cap), "cudaMallocHost (circuit batch)", err)) {
-      b.host_cap = 0;
-      return false;
-    }
-    b.host_cap = cap;
   }
   if (b.host_z_cap < b.n_z) {
     if (b.host_z) cudaFreeHost(b.host_z);
@@ -365,22 +480,52 @@ bool run_batch(Batch &b, double *out_z, cudaStream_t s, std::string &err) {
     }
     b.host_z_cap = cap;
   }
-  BHeader h{0u, nc, (uint32_t)b.ops.size(), 0u};
-  std::memcpy(b.host, &h, sizeof(h));
-  BCircuit *hc = reinterpret_cast<BCircuit *>(b.host + off_c);
-  for (uint32_t i = 0; i < nc; ++i) hc[i] = b.circs[order[i]];
-  std::memcpy(b.host + off_o, b.ops.data(), sizeof(BOp) * b.ops.size());
-  std::memcpy(b.host + off_p, b.pool.data(), b.pool.size());
+  if (!b.uploaded) {
+    std::string e1;
+    // longest first: the work counter hands them out in this order
+    std::vector<uint32_t> order(nc);
+    std::iota(order.begin(), order.end(), 0u);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](uint32_t a, uint32_t c) { return b.cost[a] > b.cost[c]; });
+    std::vector<char> tables(off_p, 0);
+    const BHeader h{0u, nc, (uint32_t)b.ops.size(), 0u};
+    std::memcpy(tables.data(), &h, sizeof(h));
+    BCircuit *hc = reinterpret_cast<BCircuit *>(tables.data() + off_c);
+    for (uint32_t i = 0; i < nc; ++i) hc[i] = b.circs[order[i]];
+    if (!b.ops.empty()) std::memcpy(tables.data() + off_o, b.ops.data(), sizeof(BOp) * b.ops.size());
+    const bool sent =
+        cuda_ok(cudaMemcpyAsync(b.dev, tables.data(), off_p, cudaMemcpyHostToDevice, s),
+                "cudaMemcpyAsync (batch upload)", err) &&
+        (b.pool.empty() || cuda_ok(cudaMemcpyAsync(b.dev + off_p, b.pool.data(), b.pool.size(),
+                                                   cudaMemcpyHostToDevice, s),
+                                   "cudaMemcpyAsync (batch matrices)", err));
+    // the tables leave this frame: wait for their copies
+    const bool there = cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (circuit batch)", e1);
+    if (sent && !there) err = e1;
+    if (!sent || !there) return false;
+    b.uploaded = true;
+  }
+  // 256 threads a CTA when every circuit is resident; shared memory for the largest
+  uint32_t state = 0;
+  bool all_resident = true;
+  for (const BCircuit &c : b.circs) {
+    if (c.resident) state = std::max(state, (c.prec ? 16u : 8u) << c.n);
+    else all_resident = false;
+  }
+  const size_t smem = kBStateOffset + state;
+  const auto kernel = all_resident ? k_circuit_batch<kBResidentThreads> : k_circuit_batch<kBThreads>;
+  const int threads = all_resident ? kBResidentThreads : kBThreads;
   int per_sm = 1;
-  if (!cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_circuit_batch, kBThreads, 0),
+  if (!cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_most()),
+               "cudaFuncSetAttribute (circuit batch)", err) ||
+      !cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor", err))
     return false;
   const uint32_t slots = (uint32_t)std::max(1, per_sm) * (uint32_t)std::max(1, cb2::sm_count());
   const unsigned grid = (unsigned)std::min<uint32_t>(nc, slots);
-  bool ok = cuda_ok(cudaMemcpyAsync(b.dev, b.host, up, cudaMemcpyHostToDevice, s),
-                    "cudaMemcpyAsync (batch upload)", err);
+  bool ok = cuda_ok(cudaMemsetAsync(b.dev, 0, sizeof(uint32_t), s), "cudaMemsetAsync (work counter)", err);
   if (ok) {
-    k_circuit_batch<<<grid, kBThreads, 0, s>>>(
+    kernel<<<grid, threads, smem, s>>>(
         reinterpret_cast<BHeader *>(b.dev), reinterpret_cast<const BCircuit *>(b.dev + off_c),
         reinterpret_cast<const BOp *>(b.dev + off_o), b.dev + off_p,
         reinterpret_cast<double *>(b.dev + off_z));
@@ -389,7 +534,7 @@ bool run_batch(Batch &b, double *out_z, cudaStream_t s, std::string &err) {
                                  cudaMemcpyDeviceToHost, s),
                  "cudaMemcpyAsync (batch <Z>)", err);
   }
-  // the pinned buffers are reused by the next run: wait for the copies either way
+  // the pinned buffer is reused by the next run: wait for the copy either way
   std::string e2;
   const bool synced = cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (circuit batch)", e2);
   if (ok && !synced) err = e2;
@@ -517,6 +662,7 @@ void cast_b200_batch_clear(void *batch) {
   b->ops.clear();
   b->pool.clear();
   b->cost.clear();
+  b->uploaded = false;
   b->n_z = 0;
 }
 

@@ -1,0 +1,498 @@
+// Gates applied to a tile of amplitudes in shared memory: device code shared by the
+// merged passes (gate_pass.cu) and the circuit batch (circuit_batch.cu), and the
+// host code that lays a gate out for it.
+//
+// complex128: a gate is a small GEMM on the FP64 tensor pipe (mma.sync m8n8k4).
+// The matrix is A, its fragments in registers for the whole gate; eight gather
+// groups are the N columns of B.  complex64: packed FP32 FMAs.
+//
+// Which tile bits the lanes walk is free: members (K order), rows and groups may
+// be taken in any order.  The host picks them so that the lanes of a shared-memory
+// wavefront fall into different bank groups under the tile's XOR swizzle (bank
+// group = XOR of the 3-bit fields of the index in 16-byte units).
+#pragma once
+
+#include "internal.hpp"
+
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+namespace cb2 {
+
+namespace {
+
+constexpr uint32_t kTileMax64 = 13, kTileMax32 = 14;  // bits of the largest tiles
+constexpr uint32_t kTileMin64 = 7;  // a 4-qubit gate and the 8 groups of a fragment
+
+// One gate of a pass.  Index contributions are swizzled tile offsets; XOR of the
+// contributions of an index's set bits is its place in shared memory.
+struct PassGateArgs {
+  uint32_t mat;          // first double of its fragments in the pool
+  uint16_t k;            // 3 or 4
+  uint16_t ld_lane[5];   // load: lane bits 0, 1 -> member bits 0, 1; 2..4 -> group bits 0..2
+  uint16_t ld_k[2];      // load: member bits 2, 3 (the k steps)
+  uint16_t st_lane[5];   // store: lane bits 0, 1 -> group bits 1, 2; 2..4 -> row bits 0..2
+  uint16_t st_row;       // store: row bit 3 (k = 4)
+  uint16_t st_col;       // store: group bit 0 (the fragment's register index)
+  uint16_t blk[kTileMax64 - 6];  // group bits 3, 4, ...
+};
+
+__host__ __device__ inline uint32_t pass_swz(uint32_t i) {
+  return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9) ^ (i >> 12)) & 7u);
+}
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ uint32_t lane_bits(const uint16_t (&c)[5], int lane) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int b = 0; b < 5; ++b)
+    if ((lane >> b) & 1) x ^= c[b];
+  return x;
+}
+
+template <int NB>
+__device__ __forceinline__ uint32_t block_bits(const PassGateArgs &g, uint32_t blk) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+    if ((blk >> b) & 1) x ^= g.blk[b];
+  return x;
+}
+
+// 4-qubit gate, three real products: S1 += c (a + b), S2 += (d - c) a,
+// S3 += (c + d) b, Re = S1 - S3, Im = S1 + S2.  (Accumulating Re and Im on top of
+// S1 saves their eight adds a block, which share the pipe, and 5% of the time at 30
+// qubits, but moves the state 10% further from its 64-bit value: not done.)
+// `m`: the gate's fragments, in global or shared memory.
+template <int W>
+__device__ __forceinline__ void pass_gate4(double2 *s, const double *mat, const PassGateArgs &g, uint32_t n_blk, int warp, int lane) {
+  double a[3][2][4];
+  const double *m = mat + lane;
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) a[p][rb][ks] = m[32 * ((p * 2 + rb) * 4 + ks)];
+  const uint32_t ld = lane_bits(g.ld_lane, lane), st = lane_bits(g.st_lane, lane);
+  for (uint32_t blk = warp; blk < n_blk; blk += W) {
+    const uint32_t bx = block_bits<kTileMax64 - 7>(g, blk);
+    double2 x[4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      x[ks] = s[bx ^ ld ^ (ks & 1 ? g.ld_k[0] : 0) ^ (ks & 2 ? g.ld_k[1] : 0)];
+    double c[3][2][2] = {};
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const double sum = x[ks].x + x[ks].y;
+#pragma unroll
+      for (int rb = 0; rb < 2; ++rb) {
+        dmma(c[0][rb], a[0][rb][ks], sum);
+        dmma(c[1][rb], a[1][rb][ks], x[ks].x);
+        dmma(c[2][rb], a[2][rb][ks], x[ks].y);
+      }
+    }
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        s[bx ^ st ^ (rb ? g.st_row : 0) ^ (i ? g.st_col : 0)] =
+            make_double2(c[0][rb][i] - c[2][rb][i], c[0][rb][i] + c[1][rb][i]);
+  }
+}
+
+// The same with four real products (Re = C a - D b, Im = D a + C b), for callers
+// whose results have always been formed that way.
+template <int W>
+__device__ __forceinline__ void pass_gate4_full(double2 *s, const double *mat, const PassGateArgs &g,
+                                                uint32_t n_blk, int warp, int lane) {
+  double c[2][4], d[2][4];
+  const double *m = mat + lane;
+#pragma unroll
+  for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      c[rb][ks] = m[32 * (rb * 4 + ks)];
+      d[rb][ks] = m[32 * (8 + rb * 4 + ks)];
+    }
+  const uint32_t ld = lane_bits(g.ld_lane, lane), st = lane_bits(g.st_lane, lane);
+  for (uint32_t blk = warp; blk < n_blk; blk += W) {
+    const uint32_t bx = block_bits<kTileMax64 - 7>(g, blk);
+    double2 x[4];
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+      x[ks] = s[bx ^ ld ^ (ks & 1 ? g.ld_k[0] : 0) ^ (ks & 2 ? g.ld_k[1] : 0)];
+    double re[2][2] = {}, im[2][2] = {};
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int rb = 0; rb < 2; ++rb) {
+        dmma(re[rb], c[rb][ks], x[ks].x);
+        dmma(im[rb], c[rb][ks], x[ks].y);
+        dmma(re[rb], -d[rb][ks], x[ks].y);
+        dmma(im[rb], d[rb][ks], x[ks].x);
+      }
+#pragma unroll
+    for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        s[bx ^ st ^ (rb ? g.st_row : 0) ^ (i ? g.st_col : 0)] = make_double2(re[rb][i], im[rb][i]);
+  }
+}
+
+// 3-qubit gate, four real products: Re = C a - D b, Im = D a + C b.  U group
+// blocks at once give the tensor pipe independent accumulators.
+template <int W, int U>
+__device__ __forceinline__ void pass_gate3_blocks(double2 *s, const double (&c)[2], const double (&d)[2],
+                                                  const PassGateArgs &g, uint32_t ld, uint32_t st,
+                                                  uint32_t blk) {
+  uint32_t bx[U];
+  double2 x[U][2];
+  double re[U][2] = {}, im[U][2] = {};
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    bx[u] = block_bits<kTileMax64 - 6>(g, blk + u * W);
+    x[u][0] = s[bx[u] ^ ld];
+    x[u][1] = s[bx[u] ^ ld ^ g.ld_k[0]];
+  }
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dmma(re[u], c[ks], x[u][ks].x);
+      dmma(im[u], c[ks], x[u][ks].y);
+      dmma(re[u], -d[ks], x[u][ks].y);
+      dmma(im[u], d[ks], x[u][ks].x);
+    }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) s[bx[u] ^ st ^ (i ? g.st_col : 0)] = make_double2(re[u][i], im[u][i]);
+}
+
+template <int W>
+__device__ __forceinline__ void pass_gate3(double2 *s, const double *mat, const PassGateArgs &g, uint32_t n_blk, int warp, int lane) {
+  const double *m = mat + lane;
+  const double c[2] = {m[0], m[32]}, d[2] = {m[64], m[96]};
+  const uint32_t ld = lane_bits(g.ld_lane, lane), st = lane_bits(g.st_lane, lane);
+  uint32_t blk = warp;
+  for (; blk + 3 * W < n_blk; blk += 4 * W)
+    pass_gate3_blocks<W, 4>(s, c, d, g, ld, st, blk);
+  for (; blk < n_blk; blk += W) pass_gate3_blocks<W, 1>(s, c, d, g, ld, st, blk);
+}
+
+constexpr uint32_t kPass32MatBytes = 3 * 256 * sizeof(float);
+
+struct PassGateArgs32 {
+  uint32_t mat;           // first float of its columns in the pool
+  uint16_t k;             // 3 or 4
+  uint16_t member[4];     // gate bits
+  uint16_t group[kTileMax32 - 3];  // group bits
+};
+
+// 16-byte units of two amplitudes; bank group = XOR of the unit's 3-bit fields.
+__host__ __device__ inline uint32_t pass_swz32(uint32_t i) {
+  const uint32_t u = i >> 1;
+  return ((u ^ (((u >> 3) ^ (u >> 6) ^ (u >> 9) ^ (u >> 12)) & 7u)) << 1) | (i & 1u);
+}
+
+template <int K>
+__device__ __forceinline__ uint32_t member_bits32(const PassGateArgs32 &g, int a) {
+  uint32_t o = 0;
+#pragma unroll
+  for (int b = 0; b < K; ++b)
+    if ((a >> b) & 1) o ^= g.member[b];
+  return o;
+}
+
+// Rows of part `half` of 1 / H of a gate for U groups at tile offsets gb.  Column c
+// of the matrix holds six floats a row pair: for three products (M3) c_0, c_1,
+// (d-c)_0, (d-c)_1, (c+d)_0, (c+d)_1; for four re_0, re_1, im_0, im_1, -im_0, -im_1.  A thread that is not `live` takes part in the barrier only.
+template <int K, int H, int U, bool M3>
+__device__ __forceinline__ void pass_groups32(float2 *s, const float *mat, const PassGateArgs32 &g,
+                                              const uint32_t (&gb)[U], uint32_t half, bool live) {
+  constexpr int D = 1 << K, P = D / 2 / H, S = M3 ? 3 : 2;  // row pairs, sums a row pair
+  const float4 *m = reinterpret_cast<const float4 *>(mat) + half * (3 * P / 2);
+  float2 acc[U][S][P];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int i = 0; i < S; ++i)
+#pragma unroll
+      for (int p = 0; p < P; ++p) acc[u][i][p] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    float2 xr[U], xi[U], xs[U];
+    const uint32_t off = member_bits32<K>(g, c);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const float2 x = s[gb[u] ^ off];
+      xr[u] = make_float2(x.x, x.x);
+      xi[u] = make_float2(x.y, x.y);
+      const float sum = x.x + x.y;
+      xs[u] = make_float2(sum, sum);
+    }
+#pragma unroll
+    for (int h = 0; h < P / 2; ++h) {  // two row pairs: three 16-byte loads
+      const float4 *mc = m + 3 * (c * (D / 4) + h);
+      const float4 m0 = mc[0], m1 = mc[1], m2 = mc[2];
+      const float2 e[2][3] = {{make_float2(m0.x, m0.y), make_float2(m0.z, m0.w), make_float2(m1.x, m1.y)},
+                              {make_float2(m1.z, m1.w), make_float2(m2.x, m2.y), make_float2(m2.z, m2.w)}};
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int p = 2 * h + q;
+          if constexpr (M3) {
+            acc[u][0][p] = __ffma2_rn(e[q][0], xs[u], acc[u][0][p]);
+            acc[u][1][p] = __ffma2_rn(e[q][1], xr[u], acc[u][1][p]);
+            acc[u][2][p] = __ffma2_rn(e[q][2], xi[u], acc[u][2][p]);
+          } else {
+            acc[u][0][p] = __ffma2_rn(e[q][2], xi[u], __ffma2_rn(e[q][0], xr[u], acc[u][0][p]));
+            acc[u][1][p] = __ffma2_rn(e[q][1], xr[u], __ffma2_rn(e[q][0], xi[u], acc[u][1][p]));
+          }
+        }
+    }
+  }
+  if constexpr (H > 1) {
+    __syncwarp();  // the partner has read this group
+    if (!live) return;
+  }
+  uint32_t top = 0;  // the half's row bits
+  if constexpr (H == 2) top = half ? g.member[K - 1] : 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      float2 re = acc[u][0][p], im = acc[u][1][p];
+      if constexpr (M3) {
+        const float2 s3 = acc[u][S - 1][p];
+        im = __fadd2_rn(re, im);
+        re = __fadd2_rn(re, make_float2(-s3.x, -s3.y));
+      }
+      s[gb[u] ^ top ^ member_bits32<K>(g, 2 * p)] = make_float2(re.x, im.x);
+      s[gb[u] ^ top ^ member_bits32<K>(g, 2 * p + 1)] = make_float2(re.y, im.y);
+    }
+}
+
+// A gate on the whole tile; H threads share a group, lane bit 4 telling them apart.
+template <int NT, int K, int H, int U, bool M3>
+__device__ __forceinline__ void pass_gate32(float2 *s, const float *mat, const PassGateArgs32 &g,
+                                            uint32_t tb) {
+  constexpr uint32_t GT = NT / H;  // groups the CTA takes at once
+  constexpr int TB = GT == 512 ? 9 : GT == 256 ? 8 : GT == 128 ? 7 : 6;
+  static_assert(GT == 1u << TB, "a power of two of groups");
+  const uint32_t half = H == 2 ? (threadIdx.x >> 4) & 1 : 0;
+  const uint32_t gt = H == 2 ? (threadIdx.x & 15) | (threadIdx.x >> 5) << 4 : threadIdx.x;
+  auto offset = [&](uint32_t group) {
+    uint32_t o = 0;
+#pragma unroll
+    for (int b = 0; b < (int)kTileMax32 - 3; ++b)
+      if ((group >> b) & 1) o ^= g.group[b];
+    return o;
+  };
+  const uint32_t groups = 1u << (tb - K), t = offset(gt);
+  if (groups >= U * GT) {
+    for (uint32_t it = 0; it < groups >> TB; it += U) {
+      uint32_t gb[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) gb[u] = t ^ offset((it + u) << TB);
+      pass_groups32<K, H, U, M3>(s, mat, g, gb, half, true);
+    }
+  } else {
+    for (uint32_t it = 0; it * GT < groups; ++it) {
+      const bool live = it * GT + gt < groups;
+      const uint32_t gb[1] = {live ? t ^ offset(it << TB) : 0};
+      if (H > 1 || live) pass_groups32<K, H, 1, M3>(s, mat, g, gb, half, live);
+    }
+  }
+}
+
+// The gate on k' = max(3, k) tile positions: positions (ascending, member bit b
+// at pos[b]) and the matrix, padded with the identity on spare positions.
+struct PlacedGate {
+  uint32_t k = 0;
+  uint32_t pos[4] = {0};
+  const double *m = nullptr;   // interleaved, 2^k x 2^k: the gate's own, or `padded`
+  std::vector<double> padded;
+};
+
+inline PlacedGate place_gate(const GateData &g, const std::vector<uint32_t> &tile_qubits) {
+  PlacedGate p;
+  auto position = [&](uint32_t q) {
+    return (uint32_t)(std::lower_bound(tile_qubits.begin(), tile_qubits.end(), q) - tile_qubits.begin());
+  };
+  uint32_t pos[4] = {0}, used = 0;
+  for (uint32_t b = 0; b < g.k; ++b) used |= 1u << (pos[b] = position(g.qubits[b]));
+  for (uint32_t c = (uint32_t)tile_qubits.size(); __builtin_popcount(used) < 3 && c-- > 0;) used |= 1u << c;
+  for (uint32_t c = 0; c < tile_qubits.size(); ++c)
+    if ((used >> c) & 1) p.pos[p.k++] = c;
+  if (p.k == g.k) {
+    p.m = g.m64.data();
+    return p;
+  }
+  const uint32_t D = 1u << p.k;
+  uint32_t gate_bit[4] = {0}, gate_mask = 0;  // bit of the padded index holding gate bit b
+  for (uint32_t b = 0; b < g.k; ++b) {
+    gate_bit[b] = (uint32_t)__builtin_popcount(used & ((1u << pos[b]) - 1));
+    gate_mask |= 1u << gate_bit[b];
+  }
+  p.padded.assign(2 * D * D, 0.0);
+  for (uint32_t r = 0; r < D; ++r)
+    for (uint32_t c = 0; c < D; ++c) {
+      if ((r ^ c) & ~gate_mask) continue;
+      uint32_t gr = 0, gc = 0;
+      for (uint32_t b = 0; b < g.k; ++b) {
+        gr |= ((r >> gate_bit[b]) & 1) << b;
+        gc |= ((c >> gate_bit[b]) & 1) << b;
+      }
+      const size_t src = 2 * (((size_t)gr << g.k) + gc), dst = 2 * ((size_t)r * D + c);
+      p.padded[dst] = g.m64[src];
+      p.padded[dst + 1] = g.m64[src + 1];
+    }
+  p.m = p.padded.data();
+  return p;
+}
+
+// How lanes walk the tile for one gate, as orders of its targets and of the
+// other positions.  Tile bit p feeds bank-group bit p % 3, so a wavefront's
+// three lane bits are conflict-free when their positions differ mod 3: members
+// 0, 1 and group bit 0 on loads, group bits 1, 2 and row bit 0 on stores.
+struct LaneOrder {
+  uint8_t member[4], row[4];      // gate bit (index into pos) by member / row bit
+  uint8_t group[kTileMax64];    // tile position by group bit
+};
+
+inline LaneOrder lane_order(const PlacedGate &p, uint32_t tb) {
+  uint32_t rest[kTileMax64], n_rest = 0, taken = 0;
+  for (uint32_t b = 0; b < p.k; ++b) taken |= 1u << p.pos[b];
+  for (uint32_t c = 0; c < tb; ++c)
+    if (!((taken >> c) & 1)) rest[n_rest++] = c;
+  auto distinct = [](uint32_t x, uint32_t y, uint32_t z) {
+    return (uint32_t)__builtin_popcount((1u << (x % 3)) | (1u << (y % 3)) | (1u << (z % 3)));
+  };
+  // the load triple, then the store triple from what is left; taking each best in
+  // turn is enough: a tile has several free positions of every class
+  uint32_t best = 0, ma = 0, mb = 1, ga = 0;
+  for (uint32_t a = 0; a < p.k && best < 3; ++a)
+    for (uint32_t b = a + 1; b < p.k && best < 3; ++b)
+      for (uint32_t x = 0; x < n_rest && best < 3; ++x) {
+        const uint32_t d = distinct(p.pos[a], p.pos[b], rest[x]);
+        if (d > best) best = d, ma = a, mb = b, ga = x;
+      }
+  uint32_t gb = n_rest, gc = n_rest, ra = 0;
+  best = 0;
+  for (uint32_t y = 0; y < n_rest && best < 3; ++y)
+    for (uint32_t z = y + 1; z < n_rest && best < 3; ++z) {
+      if (y == ga || z == ga) continue;
+      for (uint32_t r = 0; r < p.k && best < 3; ++r) {
+        const uint32_t d = distinct(rest[y], rest[z], p.pos[r]);
+        if (d > best) best = d, gb = y, gc = z, ra = r;
+      }
+    }
+  LaneOrder o{};
+  uint32_t at = 2;
+  o.member[0] = (uint8_t)ma;
+  o.member[1] = (uint8_t)mb;
+  for (uint32_t b = 0; b < p.k; ++b)
+    if (b != ma && b != mb) o.member[at++] = (uint8_t)b;
+  at = 1;
+  o.row[0] = (uint8_t)ra;
+  for (uint32_t b = 0; b < p.k; ++b)
+    if (b != ra) o.row[at++] = (uint8_t)b;
+  at = 3;
+  o.group[0] = (uint8_t)rest[ga];
+  o.group[1] = (uint8_t)rest[gb];
+  o.group[2] = (uint8_t)rest[gc];
+  for (uint32_t c = 0; c < n_rest; ++c)
+    if (c != ga && c != gb && c != gc) o.group[at++] = (uint8_t)rest[c];
+  return o;
+}
+
+// Appends a gate's A fragments to the pool (lane l holds row l / 4 and column
+// l % 4 of an 8 x 4 block) and fills its launch arguments.
+// `three`: the three-product form (4-qubit gates).
+inline void pack_gate(const PlacedGate &p, uint32_t tb, bool three, std::vector<double> &pool, PassGateArgs &out) {
+  const LaneOrder o = lane_order(p, tb);
+  const uint32_t D = 1u << p.k;
+  uint32_t row_of[16], col_of[16];
+  for (uint32_t i = 0; i < D; ++i) {
+    row_of[i] = col_of[i] = 0;
+    for (uint32_t b = 0; b < p.k; ++b)
+      if ((i >> b) & 1) {
+        row_of[i] |= 1u << o.row[b];
+        col_of[i] |= 1u << o.member[b];
+      }
+  }
+  std::memset(&out, 0, sizeof(out));
+  out.mat = (uint32_t)pool.size();
+  out.k = (uint16_t)p.k;
+  const uint32_t products = three ? 3 : 2, row_blocks = D / 8, k_steps = D / 4;
+  pool.resize(pool.size() + (size_t)products * D * D);
+  double *to = pool.data() + out.mat;
+  for (uint32_t prod = 0; prod < products; ++prod)
+    for (uint32_t rb = 0; rb < row_blocks; ++rb)
+      for (uint32_t ks = 0; ks < k_steps; ++ks)
+        for (uint32_t lane = 0; lane < 32; ++lane) {
+          const double *e = &p.m[2 * ((size_t)row_of[8 * rb + lane / 4] * D + col_of[4 * ks + lane % 4])];
+          *to++ = prod == 0 ? e[0] : !three ? e[1] : prod == 1 ? e[1] - e[0] : e[0] + e[1];
+        }
+  auto at = [](uint32_t position) { return (uint16_t)pass_swz(1u << position); };
+  for (uint32_t b = 0; b < 2; ++b) out.ld_lane[b] = at(p.pos[o.member[b]]);
+  for (uint32_t b = 0; b < 3; ++b) out.ld_lane[2 + b] = at(o.group[b]);
+  for (uint32_t b = 2; b < p.k; ++b) out.ld_k[b - 2] = at(p.pos[o.member[b]]);
+  for (uint32_t b = 0; b < 2; ++b) out.st_lane[b] = at(o.group[1 + b]);
+  for (uint32_t b = 0; b < 3; ++b) out.st_lane[2 + b] = at(p.pos[o.row[b]]);
+  if (p.k == 4) out.st_row = at(p.pos[o.row[3]]);
+  out.st_col = at(o.group[0]);
+  for (uint32_t b = 3; b < tb - p.k; ++b) out.blk[b - 3] = at(o.group[b]);
+}
+
+// A complex64 gate: its columns in row pairs appended to the pool, and the walk of
+// the tile.  A half-warp's 16 eight-byte accesses are conflict-free when one lane
+// bit is tile bit 0 and three others differ mod 3 as bits of the 16-byte unit's
+// index; when bit 0 is a target they take two wavefronts.
+inline void pack_gate32(const PlacedGate &p, uint32_t tb, bool three, std::vector<float> &pool,
+                        PassGateArgs32 &out) {
+  std::memset(&out, 0, sizeof(out));
+  out.mat = (uint32_t)pool.size();
+  out.k = (uint16_t)p.k;
+  uint32_t order[kTileMax32], n_order = 0, used = 0;
+  for (uint32_t b = 0; b < p.k; ++b) used |= 1u << p.pos[b];
+  auto take = [&](uint32_t c) {
+    order[n_order++] = c;
+    used |= 1u << c;
+  };
+  if (!(used & 1)) take(0);
+  for (uint32_t cls = 0; cls < 3; ++cls)
+    for (uint32_t c = 1 + cls; c < tb; c += 3)
+      if (!((used >> c) & 1)) {
+        take(c);
+        break;
+      }
+  for (uint32_t c = 0; c < tb; ++c)
+    if (!((used >> c) & 1)) take(c);
+  auto at = [](uint32_t position) { return (uint16_t)pass_swz32(1u << position); };
+  for (uint32_t b = 0; b < n_order; ++b) out.group[b] = at(order[b]);
+  for (uint32_t b = 0; b < p.k; ++b) out.member[b] = at(p.pos[b]);
+  const uint32_t D = 1u << p.k;
+  pool.resize(pool.size() + 3 * (size_t)D * D);
+  for (uint32_t r = 0; r < D; ++r)
+    for (uint32_t c = 0; c < D; ++c) {
+      const double re = p.m[2 * (r * D + c)], im = p.m[2 * (r * D + c) + 1];
+      float *to = &pool[out.mat + 6 * (c * (D / 2) + r / 2) + (r & 1)];
+      to[0] = (float)re;
+      to[2] = (float)(three ? im - re : im);
+      to[4] = (float)(three ? re + im : -im);
+    }
+}
+
+}  // namespace
+
+}  // namespace cb2

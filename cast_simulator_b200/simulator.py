@@ -272,7 +272,7 @@ class CircuitBatch:
                 eb, "batch_run")
         res, at = [], 0
         for n in self._sizes:
-            res.append(out[at:at + n].copy())
+            res.append(out[at:at + n])
             at += n
         return res
 
