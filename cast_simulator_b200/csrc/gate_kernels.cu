@@ -656,18 +656,6 @@ SparseLayout sparse_layout(uint32_t k, uint8_t precision, size_t nnz) {
   return l;
 }
 
-// Largest number of nonzeros in one row of the gate.
-size_t gate_row_nnz_max(const GateData &g) {
-  const size_t d = size_t(1) << g.k;
-  size_t best = 0;
-  for (size_t r = 0; r < d; ++r) {
-    size_t c = 0;
-    for (size_t e = r * d; e < (r + 1) * d; ++e) c += g.m64[2 * e] != 0.0 || g.m64[2 * e + 1] != 0.0;
-    best = std::max(best, c);
-  }
-  return best;
-}
-
 size_t gate_nnz(const GateData &g) {
   size_t nnz = 0;
   for (size_t e = 0; e < g.m64.size() / 2; ++e) nnz += g.m64[2 * e] != 0.0 || g.m64[2 * e + 1] != 0.0;
@@ -1113,6 +1101,17 @@ bool launch_gate(const GateData &g, void *sv, uint32_t n, cudaStream_t stream, s
                             : launch_sparse_t<float>(g, sv, n, t, stream, err);
   return g.precision == 1 ? launch_t<double>(g, sv, n, t, stream, err)
                           : launch_t<float>(g, sv, n, t, stream, err);
+}
+
+size_t gate_row_nnz_max(const GateData &g) {
+  const size_t d = size_t(1) << g.k;
+  size_t best = 0;
+  for (size_t r = 0; r < d; ++r) {
+    size_t c = 0;
+    for (size_t e = r * d; e < (r + 1) * d; ++e) c += g.m64[2 * e] != 0.0 || g.m64[2 * e + 1] != 0.0;
+    best = std::max(best, c);
+  }
+  return best;
 }
 
 int gate_engine(const GateData &g, uint32_t n, bool tensor, bool sparse) {

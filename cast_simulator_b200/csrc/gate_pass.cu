@@ -75,10 +75,13 @@ __global__ void __launch_bounds__(kPassThreads, 3)
   __pipeline_commit();
   __pipeline_wait_prior(0);
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the same in every lane, and known to be
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   for (uint32_t gi = 0; gi < a.n_gates; ++gi) {
     const PassGateArgs &g = a.g[gi];
     if (g.k == 4) pass_gate4<kPassWarps>(s, pool + g.mat, g, tile >> 7, warp, lane);
+    else if (g.k > 4)
+      pass_sparse<kPassWarps>(s, reinterpret_cast<const double2 *>(pool + g.mat), g.k, g.sp, a.tb, warp, lane);
     else pass_gate3<kPassWarps>(s, pool + g.mat, g, tile >> 6, warp, lane);
     __syncthreads();
   }
@@ -117,6 +120,7 @@ __global__ void __launch_bounds__(kPassThreads, 3)
   float *mat = reinterpret_cast<float *>(smem_raw);  // two gates' matrices
   float2 *s = reinterpret_cast<float2 *>(smem_raw + 2 * kPass32MatBytes);
   auto fetch_matrix = [&](uint32_t gi) {
+    if (a.g[gi].k > 4) return;  // a sparse gate's entries go to registers
     const float *from = pool + a.g[gi].mat;
     float *to = mat + (gi & 1) * (kPass32MatBytes / 4);
     for (uint32_t i = 4 * threadIdx.x; i < 3u << (2 * a.g[gi].k); i += 4 * kPassThreads)
@@ -152,6 +156,9 @@ __global__ void __launch_bounds__(kPassThreads, 3)
     const PassGateArgs32 &g = a.g[gi];
     const float *m = mat + (gi & 1) * (kPass32MatBytes / 4);
     if (g.k == 4) pass_gate32<kPassThreads, 4, 2, 2, true>(s, m, g, a.tb);
+    else if (g.k > 4)
+      pass_sparse<kPassWarps>(s, reinterpret_cast<const float2 *>(pool + g.mat), g.k, g.sp, a.tb,
+                              __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), (int)threadIdx.x & 31);
     else pass_gate32<kPassThreads, 3, 1, 4, false>(s, m, g, a.tb);
   }
   __syncthreads();
@@ -289,7 +296,8 @@ uint32_t pass_tile_bits(uint32_t n, uint8_t precision) {
 }
 
 // Which gates may share a pass, and what each saves: dense ones of up to 4 qubits
-// whose kernel nothing chose from outside.
+// and sparse ones (CSR) with few nonzeros a row, whose kernel nothing chose from
+// outside.
 //
 // A complex64 pass is bound by the FP32 pipe, so merging pays only where one-gate
 // kernels wait for memory or launches.  Not 4-qubit gates of states of 21 to 23
@@ -303,7 +311,12 @@ PassGate pass_gate_of(const GateData &g, uint32_t n) {
   PassGate p;
   for (uint32_t b = 0; b < g.k; ++b) p.qubits |= 1ull << g.qubits[b];
   const uint32_t least = g.precision ? kPassMinTile : kPass32MinTile;
-  if (n < least || g.k > 4 || g.d_tc || g.d_sparse || gate_choice_forced(g)) return p;
+  if (n < least || g.d_tc || gate_choice_forced(g)) return p;
+  if (g.d_sparse) {  // little arithmetic: a merged gate saves its whole pass
+    p.mergeable = sparse_most(g) != 0;
+    return p;
+  }
+  if (g.k > 4) return p;
   p.mergeable = g.precision || g.k < 4 || n <= 20 || n >= 24;
   p.saves = g.precision || n < 24 ? 10 : g.k == 4 ? 4 : 6;
   return p;
@@ -329,7 +342,8 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
   for (const Pass &x : p->passes)
     if (x.tile) {
       ++merged;
-      for (uint32_t i : x.gates) scalars += gates[i].k == 4 ? 3 * 256 : 3 * 64;
+      for (uint32_t i : x.gates)
+        scalars += gates[i].k > 4 ? (size_t)416 << (gates[i].k - 5) : gates[i].k == 4 ? 3 * 256 : 3 * 64;
     }
   if (f64) {
     p->pool.reserve(scalars);
@@ -355,8 +369,15 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
       a.tb = tb;
       a.n_gates = (uint32_t)x.gates.size();
       for (uint32_t j = 0; j < tb; ++j) a.stride[j] = 1ull << qubits[j];
-      for (uint32_t i = 0; i < a.n_gates; ++i)
-        pack_gate(place_gate(gates[x.gates[i]], qubits), tb, gates[x.gates[i]].k == 4, p->pool, a.g[i]);
+      for (uint32_t i = 0; i < a.n_gates; ++i) {
+        const GateData &g = gates[x.gates[i]];
+        if (g.k > 4) {
+          a.g[i].k = (uint16_t)g.k;
+          pack_sparse(g, qubits, pass_swz, p->pool, a.g[i].mat, a.g[i].sp);
+        } else {
+          pack_gate(place_gate(g, qubits), tb, g.k == 4, p->pool, a.g[i]);
+        }
+      }
     } else {
       p->args32.emplace_back();
       PassArgs32 &a = p->args32.back();
@@ -364,8 +385,15 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
       a.tb = tb;
       a.n_gates = (uint32_t)x.gates.size();
       for (uint32_t j = 0; j < tb; ++j) a.stride[j] = 1ull << qubits[j];
-      for (uint32_t i = 0; i < a.n_gates; ++i)
-        pack_gate32(place_gate(gates[x.gates[i]], qubits), tb, gates[x.gates[i]].k == 4, p->pool32, a.g[i]);
+      for (uint32_t i = 0; i < a.n_gates; ++i) {
+        const GateData &g = gates[x.gates[i]];
+        if (g.k > 4) {
+          a.g[i].k = (uint16_t)g.k;
+          pack_sparse(g, qubits, pass_swz32, p->pool32, a.g[i].mat, a.g[i].sp);
+        } else {
+          pack_gate32(place_gate(g, qubits), tb, g.k == 4, p->pool32, a.g[i]);
+        }
+      }
     }
     p->arg_of.push_back(next++);
   }

@@ -25,17 +25,28 @@ namespace {
 constexpr uint32_t kTileMax64 = 13, kTileMax32 = 14;  // bits of the largest tiles
 constexpr uint32_t kTileMin64 = 7;  // a 4-qubit gate and the 8 groups of a fragment
 
+// Sparse gates (k = 5..7, few nonzeros a row): a lane owns 2^k / 32 rows of every
+// group its warp takes.
+constexpr uint32_t kSparseMost = 8;  // rows times nonzeros a lane holds
+
+struct SparseGateArgs {
+  uint16_t most;      // entries a row is given (1, 2 or 4)
+  uint16_t full;      // every row has that many
+  uint16_t group[9];  // group bits
+};
+
 // One gate of a pass.  Index contributions are swizzled tile offsets; XOR of the
 // contributions of an index's set bits is its place in shared memory.
 struct PassGateArgs {
   uint32_t mat;          // first double of its fragments in the pool
-  uint16_t k;            // 3 or 4
+  uint16_t k;            // 3 or 4; 5..7 for a sparse gate
   uint16_t ld_lane[5];   // load: lane bits 0, 1 -> member bits 0, 1; 2..4 -> group bits 0..2
   uint16_t ld_k[2];      // load: member bits 2, 3 (the k steps)
   uint16_t st_lane[5];   // store: lane bits 0, 1 -> group bits 1, 2; 2..4 -> row bits 0..2
   uint16_t st_row;       // store: row bit 3 (k = 4)
   uint16_t st_col;       // store: group bit 0 (the fragment's register index)
   uint16_t blk[kTileMax64 - 6];  // group bits 3, 4, ...
+  SparseGateArgs sp;     // k >= 5
 };
 
 __host__ __device__ inline uint32_t pass_swz(uint32_t i) {
@@ -56,12 +67,26 @@ __device__ __forceinline__ uint32_t lane_bits(const uint16_t (&c)[5], int lane) 
   return x;
 }
 
-template <int NB>
-__device__ __forceinline__ uint32_t block_bits(const PassGateArgs &g, uint32_t blk) {
+template <int W> constexpr int log2_warps() { return W == 16 ? 4 : W == 8 ? 3 : 2; }
+
+// Group bits 3.. of block warp + W * round: the warp's share once a gate, then the
+// round's.
+template <int W>
+__device__ __forceinline__ uint32_t warp_bits(const PassGateArgs &g, int warp) {
+  static_assert(W == 1 << log2_warps<W>(), "a power of two of warps");
   uint32_t x = 0;
 #pragma unroll
-  for (int b = 0; b < NB; ++b)
-    if ((blk >> b) & 1) x ^= g.blk[b];
+  for (int b = 0; b < log2_warps<W>(); ++b)
+    if ((warp >> b) & 1) x ^= g.blk[b];
+  return x;
+}
+
+template <int W>
+__device__ __forceinline__ uint32_t round_bits(const PassGateArgs &g, uint32_t round) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int b = log2_warps<W>(); b < (int)kTileMax64 - 6; ++b)
+    if ((round >> (b - log2_warps<W>())) & 1) x ^= g.blk[b];
   return x;
 }
 
@@ -81,8 +106,9 @@ __device__ __forceinline__ void pass_gate4(double2 *s, const double *mat, const 
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) a[p][rb][ks] = m[32 * ((p * 2 + rb) * 4 + ks)];
   const uint32_t ld = lane_bits(g.ld_lane, lane), st = lane_bits(g.st_lane, lane);
-  for (uint32_t blk = warp; blk < n_blk; blk += W) {
-    const uint32_t bx = block_bits<kTileMax64 - 7>(g, blk);
+  const uint32_t wb = warp_bits<W>(g, warp);
+  for (uint32_t round = 0; round * W + warp < n_blk; ++round) {
+    const uint32_t bx = wb ^ round_bits<W>(g, round);
     double2 x[4];
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
@@ -122,8 +148,9 @@ __device__ __forceinline__ void pass_gate4_full(double2 *s, const double *mat, c
       d[rb][ks] = m[32 * (8 + rb * 4 + ks)];
     }
   const uint32_t ld = lane_bits(g.ld_lane, lane), st = lane_bits(g.st_lane, lane);
-  for (uint32_t blk = warp; blk < n_blk; blk += W) {
-    const uint32_t bx = block_bits<kTileMax64 - 7>(g, blk);
+  const uint32_t wb = warp_bits<W>(g, warp);
+  for (uint32_t round = 0; round * W + warp < n_blk; ++round) {
+    const uint32_t bx = wb ^ round_bits<W>(g, round);
     double2 x[4];
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks)
@@ -151,13 +178,13 @@ __device__ __forceinline__ void pass_gate4_full(double2 *s, const double *mat, c
 template <int W, int U>
 __device__ __forceinline__ void pass_gate3_blocks(double2 *s, const double (&c)[2], const double (&d)[2],
                                                   const PassGateArgs &g, uint32_t ld, uint32_t st,
-                                                  uint32_t blk) {
+                                                  uint32_t wb, uint32_t round) {
   uint32_t bx[U];
   double2 x[U][2];
   double re[U][2] = {}, im[U][2] = {};
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    bx[u] = block_bits<kTileMax64 - 6>(g, blk + u * W);
+    bx[u] = wb ^ round_bits<W>(g, round + u);
     x[u][0] = s[bx[u] ^ ld];
     x[u][1] = s[bx[u] ^ ld ^ g.ld_k[0]];
   }
@@ -181,19 +208,21 @@ __device__ __forceinline__ void pass_gate3(double2 *s, const double *mat, const 
   const double *m = mat + lane;
   const double c[2] = {m[0], m[32]}, d[2] = {m[64], m[96]};
   const uint32_t ld = lane_bits(g.ld_lane, lane), st = lane_bits(g.st_lane, lane);
-  uint32_t blk = warp;
-  for (; blk + 3 * W < n_blk; blk += 4 * W)
-    pass_gate3_blocks<W, 4>(s, c, d, g, ld, st, blk);
-  for (; blk < n_blk; blk += W) pass_gate3_blocks<W, 1>(s, c, d, g, ld, st, blk);
+  const uint32_t wb = warp_bits<W>(g, warp);
+  uint32_t round = 0;
+  for (; (round + 3) * W + warp < n_blk; round += 4)
+    pass_gate3_blocks<W, 4>(s, c, d, g, ld, st, wb, round);
+  for (; round * W + warp < n_blk; ++round) pass_gate3_blocks<W, 1>(s, c, d, g, ld, st, wb, round);
 }
 
 constexpr uint32_t kPass32MatBytes = 3 * 256 * sizeof(float);
 
 struct PassGateArgs32 {
   uint32_t mat;           // first float of its columns in the pool
-  uint16_t k;             // 3 or 4
+  uint16_t k;             // 3 or 4; 5..7 for a sparse gate
   uint16_t member[4];     // gate bits
   uint16_t group[kTileMax32 - 3];  // group bits
+  SparseGateArgs sp;      // k >= 5
 };
 
 // 16-byte units of two amplitudes; bank group = XOR of the unit's 3-bit fields.
@@ -290,26 +319,219 @@ __device__ __forceinline__ void pass_gate32(float2 *s, const float *mat, const P
   static_assert(GT == 1u << TB, "a power of two of groups");
   const uint32_t half = H == 2 ? (threadIdx.x >> 4) & 1 : 0;
   const uint32_t gt = H == 2 ? (threadIdx.x & 15) | (threadIdx.x >> 5) << 4 : threadIdx.x;
-  auto offset = [&](uint32_t group) {
+  auto offset = [&](uint32_t group, int from, int to) {  // group bits from .. to - 1
     uint32_t o = 0;
 #pragma unroll
     for (int b = 0; b < (int)kTileMax32 - 3; ++b)
-      if ((group >> b) & 1) o ^= g.group[b];
+      if (b >= from && b < to && ((group >> b) & 1)) o ^= g.group[b];
     return o;
   };
-  const uint32_t groups = 1u << (tb - K), t = offset(gt);
+  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0, LAST = (int)kTileMax32 - 3;
+  static_assert(U == 1 << LU, "a power of two of groups");
+  const uint32_t groups = 1u << (tb - K), t = offset(gt, 0, TB);
   if (groups >= U * GT) {
     for (uint32_t it = 0; it < groups >> TB; it += U) {
+      const uint32_t ib = t ^ offset(it << TB, TB + LU, LAST);
       uint32_t gb[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) gb[u] = t ^ offset((it + u) << TB);
+      for (int u = 0; u < U; ++u) gb[u] = ib ^ offset((uint32_t)u << TB, TB, TB + LU);
       pass_groups32<K, H, U, M3>(s, mat, g, gb, half, true);
     }
   } else {
     for (uint32_t it = 0; it * GT < groups; ++it) {
       const bool live = it * GT + gt < groups;
-      const uint32_t gb[1] = {live ? t ^ offset(it << TB) : 0};
+      const uint32_t gb[1] = {live ? t ^ offset(it << TB, TB, LAST) : 0};
       if (H > 1 || live) pass_groups32<K, H, 1, M3>(s, mat, g, gb, half, live);
+    }
+  }
+}
+
+// A sparse gate on a tile (either precision).  The entries of a lane's rows stay in
+// registers for the whole gate: per group it reads their amplitudes, waits for the
+// warp (the group is this warp's alone) and writes its rows.  An absent entry has
+// the place kNoEntry.  The same fma sequence a row as the one-gate CSR kernels.
+// A gate costs two shared-memory accesses an amplitude, so what counts is the
+// instructions around them: with the group's place formed once for U groups
+// instead of bit by bit for each, the 22-qubit QFT (CX form, complex128, 37 gates in
+// 14 passes) takes 561 us, 904 before; one gate a pass 909.  26 qubits: 19.4 ->
+// 10.8 ms in complex128, 11.3 -> 6.8 in complex64.
+constexpr uint32_t kNoEntry = 0xffffffffu;
+
+template <int ROWS, int M, int U, typename V>
+__device__ __forceinline__ void sparse_groups(V *s, const V (&m)[ROWS][M], const uint32_t (&at)[ROWS][M],
+                                              const uint32_t (&own)[ROWS], bool full,
+                                              const uint32_t (&gb)[U]) {
+  V out[U][ROWS];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      if (full) {  // every row has its M entries
+        V x = s[gb[u] ^ at[r][0]];
+        out[u][r].x = fma(m[r][0].x, x.x, -m[r][0].y * x.y);
+        out[u][r].y = fma(m[r][0].x, x.y, m[r][0].y * x.x);
+#pragma unroll
+        for (int j = 1; j < M; ++j) {
+          x = s[gb[u] ^ at[r][j]];
+          out[u][r].x = fma(m[r][j].x, x.x, fma(-m[r][j].y, x.y, out[u][r].x));
+          out[u][r].y = fma(m[r][j].x, x.y, fma(m[r][j].y, x.x, out[u][r].y));
+        }
+      } else {
+        out[u][r].x = out[u][r].y = 0;
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+          if (at[r][j] != kNoEntry) {
+            const V x = s[gb[u] ^ at[r][j]];
+            out[u][r].x = fma(m[r][j].x, x.x, fma(-m[r][j].y, x.y, out[u][r].x));
+            out[u][r].y = fma(m[r][j].x, x.y, fma(m[r][j].y, x.x, out[u][r].y));
+          }
+      }
+    }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) s[gb[u] ^ own[r]] = out[u][r];
+}
+
+template <int W, int ROWS, int M, typename V>
+__device__ __forceinline__ void pass_sparse_rows(V *s, const V *__restrict__ vals, const SparseGateArgs &g,
+                                                 uint32_t n_groups, int warp, int lane) {
+  const uint32_t *places = reinterpret_cast<const uint32_t *>(vals + 32 * ROWS * M);
+  V m[ROWS][M];
+  uint32_t at[ROWS][M], own[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+      m[r][j] = vals[32 * (r * M + j) + lane];
+      at[r][j] = places[32 * (r * M + j) + lane];
+    }
+    own[r] = places[32 * (ROWS * M + r) + lane];
+  }
+  // group bits: the warp, then the U groups taken at once, then the rounds
+  constexpr int LU = ROWS * M >= 8 ? 0 : ROWS * M >= 4 ? 1 : 2, U = 1 << LU;
+  constexpr int LW = log2_warps<W>();
+  uint32_t wb = 0;
+#pragma unroll
+  for (int b = 0; b < LW; ++b)
+    if ((warp >> b) & 1) wb ^= g.group[b];
+  if (n_groups >= (uint32_t)(U * W)) {
+    for (uint32_t it = 0; it < n_groups / (U * W); ++it) {
+      uint32_t ib = wb;
+#pragma unroll
+      for (int b = LW + LU; b < 9; ++b)
+        if ((it >> (b - LW - LU)) & 1) ib ^= g.group[b];
+      uint32_t gb[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        gb[u] = ib;
+#pragma unroll
+        for (int b = 0; b < LU; ++b)
+          if ((u >> b) & 1) gb[u] ^= g.group[LW + b];
+      }
+      sparse_groups<ROWS, M, U>(s, m, at, own, g.full, gb);
+    }
+  } else {
+    for (uint32_t group = warp; group < n_groups; group += W) {
+      uint32_t gb[1] = {wb};
+#pragma unroll
+      for (int b = LW; b < 9; ++b)
+        if ((group >> b) & 1) gb[0] ^= g.group[b];
+      sparse_groups<ROWS, M, 1>(s, m, at, own, g.full, gb);
+    }
+  }
+}
+
+template <int W, typename V>
+__device__ __forceinline__ void pass_sparse(V *s, const V *__restrict__ vals, uint32_t k,
+                                            const SparseGateArgs &g, uint32_t tb, int warp, int lane) {
+  const uint32_t n = 1u << (tb - k);
+  if (k == 5) {
+    if (g.most == 1) pass_sparse_rows<W, 1, 1>(s, vals, g, n, warp, lane);
+    else pass_sparse_rows<W, 1, 4>(s, vals, g, n, warp, lane);
+  } else if (k == 6) {
+    if (g.most == 1) pass_sparse_rows<W, 2, 1>(s, vals, g, n, warp, lane);
+    else pass_sparse_rows<W, 2, 4>(s, vals, g, n, warp, lane);
+  } else {
+    if (g.most == 1) pass_sparse_rows<W, 4, 1>(s, vals, g, n, warp, lane);
+    else pass_sparse_rows<W, 4, 2>(s, vals, g, n, warp, lane);
+  }
+}
+
+// Entries a row of a sparse gate is given in its tile form, 0 when it has too many
+// nonzeros for one.
+inline uint32_t sparse_most(const GateData &g) {
+  const size_t most = gate_row_nnz_max(g);
+  const uint32_t rows = 1u << (g.k - 5), cap = g.k == 7 ? 2 : 4;
+  if (most > cap || rows * cap > kSparseMost) return 0;
+  return most <= 1 ? 1 : cap;
+}
+
+// A sparse gate's entries appended to the pool (T: its scalars) and its walk; `swz`
+// maps a tile index to its place.
+template <typename T, typename S>
+inline void pack_sparse(const GateData &g, const std::vector<uint32_t> &tile_qubits, S swz,
+                        std::vector<T> &pool, uint32_t &mat, SparseGateArgs &out) {
+  const uint32_t D = 1u << g.k, tb = (uint32_t)tile_qubits.size(), rows = D / 32;
+  const uint32_t M = out.most = (uint16_t)sparse_most(g);
+  uint32_t pos[kMaxGateQubits], taken = 0;
+  for (uint32_t b = 0; b < g.k; ++b) {
+    pos[b] = (uint32_t)(std::lower_bound(tile_qubits.begin(), tile_qubits.end(), g.qubits[b]) -
+                        tile_qubits.begin());
+    taken |= 1u << pos[b];
+  }
+  uint32_t at = 0;
+  for (uint32_t c = 0; c < tb; ++c)
+    if (!((taken >> c) & 1)) out.group[at++] = (uint16_t)swz(1u << c);
+  while (pool.size() % 4) pool.push_back(T(0));  // 16-byte aligned
+  mat = (uint32_t)pool.size();
+  const size_t entries = 32 * (size_t)rows * M;
+  pool.resize(pool.size() + 2 * entries + (entries + D) * sizeof(uint32_t) / sizeof(T));
+  T *vals = pool.data() + mat;
+  uint32_t *places = reinterpret_cast<uint32_t *>(vals + 2 * entries);
+  for (size_t e = 0; e < entries; ++e) places[e] = kNoEntry;
+  uint32_t member[1u << kMaxGateQubits];  // place of a member in its group
+  for (uint32_t i = 0; i < D; ++i) {
+    member[i] = 0;
+    for (uint32_t b = 0; b < g.k; ++b)
+      if ((i >> b) & 1) member[i] ^= swz(1u << pos[b]);
+  }
+  uint8_t cols[1u << kMaxGateQubits][4], n_cols[1u << kMaxGateQubits];
+  out.full = 1;
+  for (uint32_t r = 0; r < D; ++r) {
+    n_cols[r] = 0;
+    for (uint32_t c = 0; c < D; ++c)
+      if (g.m64[2 * ((size_t)r * D + c)] != 0.0 || g.m64[2 * ((size_t)r * D + c) + 1] != 0.0)
+        cols[r][n_cols[r]++] = (uint8_t)c;
+    if (n_cols[r] != M) out.full = 0;
+  }
+  // Rows are dealt to lanes wavefront by wavefront (8 lanes of 16-byte amplitudes or
+  // 16 of 8-byte ones), each time the row whose own place and inputs meet the fewest
+  // taken banks: a permutation's rows and columns rarely suit the same plain order.
+  constexpr uint32_t WF = 128 / (2 * sizeof(T));
+  bool dealt[1u << kMaxGateQubits] = {};
+  for (uint32_t first = 0; first < D; first += WF) {
+    uint8_t used[1 + 4][16] = {};  // own place, then each entry's; by bank slot
+    for (uint32_t i = first; i < first + WF; ++i) {
+      uint32_t row = D, least = ~0u;
+      for (uint32_t r = 0; r < D && least; ++r) {
+        if (dealt[r]) continue;
+        uint32_t clash = used[0][member[r] % WF];
+        for (uint32_t j = 0; j < n_cols[r]; ++j) clash += used[1 + j][member[cols[r][j]] % WF];
+        if (clash < least) least = clash, row = r;
+      }
+      dealt[row] = true;
+      ++used[0][member[row] % WF];
+      places[entries + i] = member[row];
+      for (uint32_t j = 0; j < n_cols[row]; ++j) {
+        const uint32_t c = cols[row][j];
+        ++used[1 + j][member[c] % WF];
+        const size_t e = 32 * ((size_t)(i / 32) * M + j) + i % 32, from = 2 * ((size_t)row * D + c);
+        vals[2 * e] = (T)g.m64[from];
+        vals[2 * e + 1] = (T)g.m64[from + 1];
+        places[e] = member[c];
+      }
     }
   }
 }

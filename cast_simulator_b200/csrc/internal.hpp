@@ -68,6 +68,7 @@ bool launch_gate(const GateData &g, void *sv, uint32_t n, cudaStream_t stream, s
 // snapping) run on the CSR kernel instead of the dense ones; upload_sparse
 // fills g.d_sparse.  free_gate_device releases every device copy of a gate.
 bool sparse_gate(const GateData &g);
+size_t gate_row_nnz_max(const GateData &g);  // largest number of nonzeros in a row
 
 // The kernel family a gate runs on (the same decisions launch_gate takes):
 // `tensor` = the gate carries a tensor-core operand, `sparse` = a CSR table.

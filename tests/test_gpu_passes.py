@@ -51,3 +51,40 @@ def test_program_matches_oracle(n, widths, graph, prec):
     # 24 unitary gates: each adds at most a few units of 2^k roundings
     bound = 24 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
     assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
+
+
+def _sparse_gate(n, k, per_row, rng):
+    """A unitary of 2^k with per_row nonzeros a row: blocks times a permutation."""
+    d = 1 << k
+    m = np.zeros((d, d), dtype=np.complex128)
+    for b in range(0, d, per_row):
+        q, _ = np.linalg.qr(rng.standard_normal((per_row, per_row)) + 1j * rng.standard_normal((per_row, per_row)))
+        m[b:b + per_row, b:b + per_row] = q
+    m = m[rng.permutation(d)][:, rng.permutation(d)]
+    qs = np.sort(rng.choice(n, size=k, replace=False))
+    if rng.random() < 0.5:
+        q0 = int(rng.integers(0, n - k + 1))
+        qs = np.arange(q0, q0 + k)
+    return T.QuantumGate(m, [int(q) for q in qs])
+
+
+@pytest.mark.parametrize("n", [7, 9, 10, 12, 13, 16, 19, 21])
+@pytest.mark.parametrize("prec", [CudaPrecision.F64, CudaPrecision.F32])
+def test_sparse_gates_in_passes(n, prec):
+    rng = np.random.default_rng(n)
+    psi = O.random_state(n, n)
+    tol = 1e-12 if prec == CudaPrecision.F64 else 1e-6
+    prog, want = GateProgram(prec, n, tol, tol), psi.copy()
+    for i in range(18):
+        # 5 to 7 qubits with 1 to 8 nonzeros a row (7 qubits: up to 2 merge, more run alone)
+        k = 5 + i % 3
+        g = (T.QuantumGate.random_unitary([int(q) for q in rng.choice(n, size=3, replace=False)], rng)
+             if i % 6 == 5 else _sparse_gate(n, min(k, n), (1, 2, 1, 4, 8)[i % 5], rng))
+        prog.add(g.matrix(), g.qubits())
+        O.apply_gate(want, g.matrix(), g.qubits())
+    sv, st = CudaStatevector(n, prec), Stream()
+    sv.upload(psi)
+    prog.run(sv, st)
+    st.sync()
+    bound = 18 * 8 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
+    assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
