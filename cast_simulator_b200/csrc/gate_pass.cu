@@ -159,7 +159,8 @@ __global__ void __launch_bounds__(kPassThreads, 3)
     else if (g.k > 4)
       pass_sparse<kPassWarps>(s, reinterpret_cast<const float2 *>(pool + g.mat), g.k, g.sp, a.tb,
                               __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), (int)threadIdx.x & 31);
-    else pass_gate32<kPassThreads, 3, 1, 4, false>(s, m, g, a.tb);
+    else if (g.k == 3) pass_gate32<kPassThreads, 3, 1, 4, false>(s, m, g, a.tb);
+    else pass_gate32<kPassThreads, 2, 1, 4, false>(s, m, g, a.tb);
   }
   __syncthreads();
 #pragma unroll 8
@@ -375,7 +376,7 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
           a.g[i].k = (uint16_t)g.k;
           pack_sparse(g, qubits, pass_swz, p->pool, a.g[i].mat, a.g[i].sp);
         } else {
-          pack_gate(place_gate(g, qubits), tb, g.k == 4, p->pool, a.g[i]);
+          pack_gate(place_gate(g, qubits, 3), tb, g.k == 4, p->pool, a.g[i]);
         }
       }
     } else {
@@ -391,7 +392,7 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
           a.g[i].k = (uint16_t)g.k;
           pack_sparse(g, qubits, pass_swz32, p->pool32, a.g[i].mat, a.g[i].sp);
         } else {
-          pack_gate32(place_gate(g, qubits), tb, g.k == 4, p->pool32, a.g[i]);
+          pack_gate32(place_gate(g, qubits, 2), tb, g.k == 4, p->pool32, a.g[i]);
         }
       }
     }

@@ -219,9 +219,9 @@ constexpr uint32_t kPass32MatBytes = 3 * 256 * sizeof(float);
 
 struct PassGateArgs32 {
   uint32_t mat;           // first float of its columns in the pool
-  uint16_t k;             // 3 or 4; 5..7 for a sparse gate
+  uint16_t k;             // 2..4; 5..7 for a sparse gate
   uint16_t member[4];     // gate bits
-  uint16_t group[kTileMax32 - 3];  // group bits
+  uint16_t group[kTileMax32 - 2];  // group bits (a 2-qubit gate has the most)
   SparseGateArgs sp;      // k >= 5
 };
 
@@ -322,11 +322,11 @@ __device__ __forceinline__ void pass_gate32(float2 *s, const float *mat, const P
   auto offset = [&](uint32_t group, int from, int to) {  // group bits from .. to - 1
     uint32_t o = 0;
 #pragma unroll
-    for (int b = 0; b < (int)kTileMax32 - 3; ++b)
+    for (int b = 0; b < (int)kTileMax32 - 2; ++b)
       if (b >= from && b < to && ((group >> b) & 1)) o ^= g.group[b];
     return o;
   };
-  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0, LAST = (int)kTileMax32 - 3;
+  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0, LAST = (int)kTileMax32 - 2;
   static_assert(U == 1 << LU, "a power of two of groups");
   const uint32_t groups = 1u << (tb - K), t = offset(gt, 0, TB);
   if (groups >= U * GT) {
@@ -536,7 +536,7 @@ inline void pack_sparse(const GateData &g, const std::vector<uint32_t> &tile_qub
   }
 }
 
-// The gate on k' = max(3, k) tile positions: positions (ascending, member bit b
+// The gate on k' = max(least, k) tile positions: positions (ascending, member bit b
 // at pos[b]) and the matrix, padded with the identity on spare positions.
 struct PlacedGate {
   uint32_t k = 0;
@@ -545,14 +545,14 @@ struct PlacedGate {
   std::vector<double> padded;
 };
 
-inline PlacedGate place_gate(const GateData &g, const std::vector<uint32_t> &tile_qubits) {
+inline PlacedGate place_gate(const GateData &g, const std::vector<uint32_t> &tile_qubits, uint32_t least) {
   PlacedGate p;
   auto position = [&](uint32_t q) {
     return (uint32_t)(std::lower_bound(tile_qubits.begin(), tile_qubits.end(), q) - tile_qubits.begin());
   };
   uint32_t pos[4] = {0}, used = 0;
   for (uint32_t b = 0; b < g.k; ++b) used |= 1u << (pos[b] = position(g.qubits[b]));
-  for (uint32_t c = (uint32_t)tile_qubits.size(); __builtin_popcount(used) < 3 && c-- > 0;) used |= 1u << c;
+  for (uint32_t c = (uint32_t)tile_qubits.size(); (uint32_t)__builtin_popcount(used) < least && c-- > 0;) used |= 1u << c;
   for (uint32_t c = 0; c < tile_qubits.size(); ++c)
     if ((used >> c) & 1) p.pos[p.k++] = c;
   if (p.k == g.k) {

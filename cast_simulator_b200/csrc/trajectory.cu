@@ -9,7 +9,13 @@
 //    complex64 statevector lives in a per-CTA slice of a workspace in global
 //    memory (148 CTAs x 512 KiB = 74 MiB at 16 qubits, resident in the 126 MB
 //    L2); the CTA loops over trajectories blockIdx.x, blockIdx.x + gridDim.x, ...
-//  * GATE ops are fused unitary blocks (k <= 4) applied in place;
+//  * GATE ops are fused unitary blocks (k <= 4).  A run of them up to the next DAMP
+//    or CHAN op is a segment: when none of its ERR sites fires (their draws do not
+//    depend on the state), its blocks share passes over the state as a gate
+//    program's gates do (pass_plan.hpp, gate_tile.cuh), tiles of up to 2^13
+//    amplitudes in shared memory with the next tile's copy in flight; otherwise, and
+//    for programs without such segments, the blocks are applied one after the other
+//    in place;
 //  * ERR ops are state-independent Pauli errors (depolarizing): a Philox draw
 //    decides; when one fires, the Pauli propagated to the end of its fused
 //    block (U P U^dagger, precomputed on the host) is applied as a gate;
@@ -25,7 +31,8 @@
 // bitstring sampled from |psi|^2.  Branch sums, renormalisation factors and the
 // final reductions are FP64; amplitudes and gate arithmetic are FP32.
 #include "../../include/cast_b200.h"
-#include "internal.hpp"
+#include "gate_tile.cuh"
+#include "pass_plan.hpp"
 #include "philox.cuh"
 
 #include <algorithm>
@@ -34,6 +41,8 @@
 #include <map>
 #include <mutex>
 #include <vector>
+
+#include <cuda_pipeline.h>
 
 namespace {
 
@@ -59,6 +68,33 @@ struct TOp {
   float prob;      // ERR: firing probability
   float gamma;     // DAMP: damping rate
   float sgamma;    // GATE stats: damping rate of that op
+  uint32_t seg;    // GATE: 1 + the segment that starts here, or 0
+};
+
+// A run of GATE ops (and the ERR ops that follow them) grouped into passes.
+struct TSeg {
+  uint32_t end_op;           // first op after it
+  uint32_t pass0, n_passes;
+  uint32_t err0, n_err;      // its ERR ops, in order (entries of the site list)
+  uint32_t stats, smask;     // the DAMP op behind it, if any (as TOp)
+  float sgamma;
+};
+struct TSegPass {
+  uint32_t tb, n_gates;
+  uint32_t gate0;            // first entry of the gate list
+  uint32_t mat, mat_bytes;   // its gates' matrices, one after the other
+  uint32_t stride[13];       // tile bit -> amplitude stride
+};
+constexpr uint32_t kSegMaxTile = 13, kSegLow = 4;
+constexpr uint32_t kSegMinQubits = 8;  // below, a pass costs what its gates do (6 qubits: 1.26 against 1.20 ms)
+
+struct TSegs {  // device arrays of a program's segments
+  const TSeg *segs;
+  const TSegPass *passes;
+  const cb2::PassGateArgs32 *gates;
+  const uint32_t *sites;     // op index of every ERR op of a segment
+  const float *mats;
+  uint32_t mat_cap;          // bytes kept for a pass's matrices
 };
 
 struct TRun {  // device-resident, rewritten before each launch
@@ -81,6 +117,7 @@ struct Shared {
   float dtab[kTrajMaxQubits + 1];  // pending diagonal: scale * s^popc
   double stab[kTrajMaxQubits + 1]; // damping weights (1 - g)^popc for the sums
   uint32_t pmask;
+  uint32_t pick;  // chunk of the sampled bitstring
   int pend;
 };
 
@@ -91,6 +128,9 @@ __device__ __forceinline__ float2 cmul_add(float2 m, float2 x, float2 acc) {
   acc.y = fmaf(m.y, x.x, acc.y);
   return acc;
 }
+
+// Shared memory kept for a pass's gate arguments.
+constexpr uint32_t kSegArgBytes = (cb2::kMaxPassGates * sizeof(cb2::PassGateArgs32) + 15) & ~15u;
 
 // The device side of one trajectory, for CTAs of NT threads.  512-thread CTAs
 // get 128 registers a thread, so the fused gates run without spills (the passes
@@ -422,39 +462,184 @@ struct Traj {
     set_pending(S, 0, 0.0, t > 0 ? 1.0 / sqrt(t) : 1.0);
   }
 
+  // The passes of a segment.  A block in place costs its loads' latency through L2
+  // and a matrix entry from shared memory for every four FMAs: 27 us a block of a
+  // 16-qubit state, whose arithmetic takes 4 to 9.  2048 trajectories of 16 qubits and
+  // depth 30 (fused at 3): 87.5 -> 73 ms; 18 qubits, depth 20 (296): 54 -> 37 ms; 12
+  // qubits (2048): 5.8 -> 4.8 ms.  What is left is latency: 16 warps issue 0.41
+  // instructions a clock and scheduler, waiting for shared memory and for each other.
+  // The first applies the pending diagonal as its tiles
+  // arrive, the last sums t and d (as gate_pass does) as its tiles leave.  Two tile
+  // buffers: the next tile is copied in while this one is computed.
+  static __device__ __noinline__ void run_segment(float2 *sv, uint32_t n, const TSeg &seg, const TSegs &G,
+                                                  unsigned char *smem, const Shared &S, double &t,
+                                                  double &d) {
+    float *const mats = reinterpret_cast<float *>(smem);
+    cb2::PassGateArgs32 *const args = reinterpret_cast<cb2::PassGateArgs32 *>(smem + G.mat_cap);
+    const bool pend = S.pend != 0;
+    const uint32_t pmask = S.pmask;
+    for (uint32_t pi = 0; pi < seg.n_passes; ++pi) {
+      const TSegPass &P = G.passes[seg.pass0 + pi];
+      const uint32_t tb = P.tb, tile = 1u << tb, n_tiles = 1u << (n - tb), n_gates = P.n_gates;
+      float2 *const buf = reinterpret_cast<float2 *>(smem + G.mat_cap + kSegArgBytes);
+      for (uint32_t i = threadIdx.x; i < n_gates * sizeof(cb2::PassGateArgs32) / 4; i += NT)
+        reinterpret_cast<uint32_t *>(args)[i] = reinterpret_cast<const uint32_t *>(G.gates + P.gate0)[i];
+      for (uint32_t i = 16 * threadIdx.x; i < P.mat_bytes; i += 16 * NT)
+        __pipeline_memcpy_async(smem + i, reinterpret_cast<const char *>(G.mats + P.mat) + i, 16);
+      // pairs of amplitudes: tile bits 1 .. kTLogThreads are the thread index, the
+      // bits above the rounds; where each starts, and the tiles' first amplitudes in
+      // ascending order of the other qubits
+      constexpr uint32_t R = (1u << kSegMaxTile) / (2 * NT);
+      uint32_t at[R], tmask = 0;
+      for (uint32_t b = 0; b < tb; ++b) tmask |= P.stride[b];
+      uint32_t off = 0;
+#pragma unroll
+      for (uint32_t b = 0; b < kTLogThreads; ++b)
+        if (b + 1 < tb && ((threadIdx.x >> b) & 1)) off += P.stride[b + 1];
+#pragma unroll
+      for (uint32_t u = 0; u < R; ++u) {
+        at[u] = off;
+#pragma unroll
+        for (uint32_t b = kTLogThreads + 1; b < kSegMaxTile; ++b)
+          if (b < tb && ((u >> (b - kTLogThreads - 1)) & 1)) at[u] += P.stride[b];
+      }
+      const uint32_t rounds = 2 * threadIdx.x < tile ? (tile + 2 * NT - 1) / (2 * NT) : 0;
+      uint32_t base = 0, next = 0;  // of this tile and the next one to fetch
+      auto fetch = [&](float2 *to) {
+#pragma unroll
+        for (uint32_t u = 0; u < R; ++u)
+          if (u < rounds)
+            __pipeline_memcpy_async(&to[cb2::pass_swz32(2 * (threadIdx.x + u * NT))], &sv[next + at[u]], 16);
+        next = ((next | tmask) + 1) & ~tmask;
+      };
+      fetch(buf);
+      __pipeline_commit();
+      for (uint32_t tl = 0; tl < n_tiles; ++tl) {
+        float2 *s = buf + (tl & 1) * tile;
+        if (tl + 1 < n_tiles) fetch(buf + ((tl + 1) & 1) * tile);
+        __pipeline_commit();
+        __pipeline_wait_prior(1);
+        if (pend && pi == 0) {  // a thread scales what it copied
+#pragma unroll
+          for (uint32_t u = 0; u < R; ++u)
+            if (u < rounds) {
+              const uint32_t i = base + at[u];
+              float4 *v = reinterpret_cast<float4 *>(&s[cb2::pass_swz32(2 * (threadIdx.x + u * NT))]);
+              const float f0 = S.dtab[__popc(i & pmask)], f1 = S.dtab[__popc((i | 1) & pmask)];
+              float4 x = *v;
+              x.x *= f0;
+              x.y *= f0;
+              x.z *= f1;
+              x.w *= f1;
+              *v = x;
+            }
+        }
+        __syncthreads();
+        const float *m = mats;
+        for (uint32_t gi = 0; gi < n_gates; ++gi) {
+          const cb2::PassGateArgs32 &g = args[gi];
+          if (g.k == 4) {
+            cb2::pass_gate32<NT, 4, 2, 2, false>(s, m, g, tb);
+            m += 3 * 256;
+          } else if (g.k == 3) {
+            cb2::pass_gate32<NT, 3, 1, 2, false>(s, m, g, tb);
+            m += 3 * 64;
+          } else {
+            cb2::pass_gate32<NT, 2, 1, 4, false>(s, m, g, tb);
+            m += 3 * 16;
+          }
+          __syncthreads();
+        }
+        const bool sum = seg.stats && pi + 1 == seg.n_passes;
+#pragma unroll
+        for (uint32_t u = 0; u < R; ++u)
+          if (u < rounds) {
+            const uint32_t i = base + at[u];
+            const float4 v = *reinterpret_cast<const float4 *>(&s[cb2::pass_swz32(2 * (threadIdx.x + u * NT))]);
+            *reinterpret_cast<float4 *>(&sv[i]) = v;
+            if (sum) {
+              const double p0 = (double)v.x * v.x + (double)v.y * v.y;
+              const double p1 = (double)v.z * v.z + (double)v.w * v.w;
+              t += p0 + p1;
+              d += p0 * S.stab[__popc(i & seg.smask)] + p1 * S.stab[__popc((i | 1) & seg.smask)];
+            }
+          }
+        base = ((base | tmask) + 1) & ~tmask;
+        __syncthreads();  // the buffer is read out, the state written
+      }
+    }
+  }
+
   // End of a trajectory: <Z_q> for every qubit and one sampled bitstring.
   static __device__ __noinline__ void finish(float2 *sv, uint32_t n, Shared &S, double *csum, uint64_t seed,
                                       uint32_t traj, double *z_row, uint32_t *sample_slot) {
-    {
-      double t, a, b;
-      stats_pass(sv, n, S, 0, 0.0, 0, t, a, b);  // materialise the pending diagonal
-    }
     const uint32_t N = 1u << n;
     const uint32_t c = n > kTLogThreads ? n - kTLogThreads : 0;  // bits inside a thread's chunk
     const uint32_t chunk = 1u << c;
-    const bool active = (threadIdx.x << c) < N;
-    const uint32_t base = threadIdx.x << c;
-    double my = 0;
-    if (active)
-      for (uint32_t i = 0; i < chunk; ++i) {
-        const float2 v = sv[base + i];
-        my += (double)v.x * v.x + (double)v.y * v.y;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // The pending diagonal stays pending: every read below applies it.
+    if (c >= 5) {
+      // one coalesced pass: a warp sums a chunk, so a lane's place in it is fixed and
+      // its total serves the five lowest qubits (not a chunk a thread, which reads
+      // 32 lines a warp, again for every three of its qubits)
+      constexpr int HIGH = (int)kTrajMaxQubits - (int)kTLogThreads - 5;
+      double tot = 0, high[HIGH];
+#pragma unroll
+      for (int q = 0; q < HIGH; ++q) high[q] = 0;
+      for (uint32_t ch = warp; ch < (uint32_t)NT; ch += NT / 32) {
+        double sum = 0;
+        for (uint32_t j = 0; j < chunk >> 5; ++j) {
+          const float2 v = pend_load(sv, (ch << c) + (j << 5) + lane, S);
+          const double p = (double)v.x * v.x + (double)v.y * v.y;
+          sum += p;
+#pragma unroll
+          for (int q = 0; q < HIGH; ++q)
+            if ((j >> q) & 1) high[q] += p;
+        }
+        tot += sum;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+        if (lane == 0) csum[ch] = sum;
       }
-    csum[threadIdx.x] = my;
-    __syncthreads();
-    // qubits inside a chunk, three per block reduction
-    for (uint32_t q0 = 0; q0 < c; q0 += 3) {
-      double acc[3] = {0, 0, 0};
+      for (uint32_t q0 = 0; q0 < c; q0 += 3) {
+        double acc[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int q = (int)q0 + j;
+          acc[j] = q < 5 && ((lane >> q) & 1) ? tot : 0.0;
+#pragma unroll
+          for (int h = 0; h < HIGH; ++h)
+            if (q == 5 + h) acc[j] = high[h];
+        }
+        block_sum3(S, acc[0], acc[1], acc[2]);
+        if (threadIdx.x < 3 && q0 + threadIdx.x < c) z_row[q0 + threadIdx.x] = acc[threadIdx.x];
+      }
+    } else {
+      const bool active = (threadIdx.x << c) < N;
+      const uint32_t base = threadIdx.x << c;
+      double my = 0;
       if (active)
         for (uint32_t i = 0; i < chunk; ++i) {
-          const float2 v = sv[base + i];
-          const double p = (double)v.x * v.x + (double)v.y * v.y;
-          for (uint32_t j = 0; j < 3; ++j)
-            if (q0 + j < c && ((i >> (q0 + j)) & 1)) acc[j] += p;
+          const float2 v = pend_load(sv, base + i, S);
+          my += (double)v.x * v.x + (double)v.y * v.y;
         }
-      block_sum3(S, acc[0], acc[1], acc[2]);
-      if (threadIdx.x < 3 && q0 + threadIdx.x < c) z_row[q0 + threadIdx.x] = acc[threadIdx.x];
+      csum[threadIdx.x] = my;
+      __syncthreads();
+      // qubits inside a chunk, three per block reduction
+      for (uint32_t q0 = 0; q0 < c; q0 += 3) {
+        double acc[3] = {0, 0, 0};
+        if (active)
+          for (uint32_t i = 0; i < chunk; ++i) {
+            const float2 v = pend_load(sv, base + i, S);
+            const double p = (double)v.x * v.x + (double)v.y * v.y;
+            for (uint32_t j = 0; j < 3; ++j)
+              if (q0 + j < c && ((i >> (q0 + j)) & 1)) acc[j] += p;
+          }
+        block_sum3(S, acc[0], acc[1], acc[2]);
+        if (threadIdx.x < 3 && q0 + threadIdx.x < c) z_row[q0 + threadIdx.x] = acc[threadIdx.x];
+      }
     }
+    __syncthreads();
     // qubits that index the threads: thread j sums the chunk sums with bit j set
     const uint32_t nthr = N >> c;
     if (threadIdx.x < n - c) {
@@ -463,6 +648,7 @@ struct Traj {
         if ((tt >> threadIdx.x) & 1) x += csum[tt];
       z_row[c + threadIdx.x] = x;
     }
+    __syncthreads();  // the sums over csum are done
     if (threadIdx.x == 0) {
       double tot = 0;
       for (uint32_t tt = 0; tt < nthr; ++tt) tot += csum[tt];
@@ -480,18 +666,32 @@ struct Traj {
         if (acc + csum[tt] > target) break;
         acc += csum[tt];
       }
-      acc = acc_t;
-      if (tsel == nthr) tsel = 0;  // an all-zero state (cannot arise from normalised branches)
-      uint32_t isel = tsel << c;
-      for (uint32_t i = 0; i < chunk; ++i) {
-        const float2 v = sv[(tsel << c) + i];
-        const double p = (double)v.x * v.x + (double)v.y * v.y;
-        if (p > 0) isel = (tsel << c) + i;
-        acc += p;
-        if (acc > target) break;
-      }
-      if (sample_slot) *sample_slot = isel;
+      S.vals[0] = target;
+      S.vals[1] = acc_t;
+      S.pick = tsel == nthr ? 0 : tsel;  // an all-zero state (cannot arise from normalised branches)
     }
+    __syncthreads();
+    const uint32_t first = S.pick << c;
+    // the chosen chunk's probabilities, NT at a time
+    double acc = S.vals[1];
+    const double target = S.vals[0];
+    uint32_t isel = first;
+    for (uint32_t part = 0; part < chunk; part += NT) {
+      const uint32_t len = min(chunk - part, (uint32_t)NT);
+      if (threadIdx.x < len) {
+        const float2 v = pend_load(sv, first + part + threadIdx.x, S);
+        csum[threadIdx.x] = (double)v.x * v.x + (double)v.y * v.y;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0)
+        for (uint32_t i = 0; i < len && !(acc > target); ++i) {
+          const double p = csum[i];
+          if (p > 0) isel = first + part + i;
+          acc += p;
+        }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0 && sample_slot) *sample_slot = isel;
     __syncthreads();
     const double tot = S.vals[3];
     if (threadIdx.x < n) {
@@ -506,7 +706,9 @@ template <int NT>
 __global__ void __launch_bounds__(NT, 1)
     k_trajectories(const TOp *__restrict__ ops, uint32_t n_ops, const float2 *__restrict__ pool,
                    float2 *__restrict__ ws, uint32_t n, const TRun *__restrict__ run,
-                   double *__restrict__ out_z, uint32_t *__restrict__ out_sample) {
+                   double *__restrict__ out_z, uint32_t *__restrict__ out_sample,
+                   const __grid_constant__ TSegs segs) {
+  extern __shared__ __align__(16) unsigned char seg_smem[];
   __shared__ Shared S;
   __shared__ float2 Msm[1 << (2 * kTrajMaxGate)];
   __shared__ double csum[NT];
@@ -526,6 +728,31 @@ __global__ void __launch_bounds__(NT, 1)
     double T = 1.0, Dd = 1.0;
     for (uint32_t oi = 0; oi < n_ops; ++oi) {
       const TOp op = ops[oi];
+      if constexpr (NT == kTMinThreads) {
+        if (op.seg && segs.segs) {
+          const TSeg seg = segs.segs[op.seg - 1];
+          int fired = 0;
+          for (uint32_t e = threadIdx.x; e < seg.n_err; e += NT)
+            fired |= philox_uniform(seed, traj, ev + e) < (double)ops[segs.sites[seg.err0 + e]].prob;
+          if (!__syncthreads_or(fired)) {
+            if (seg.stats) Tr::fill_stab(S, (double)seg.sgamma);
+            double t = 0, d = 0, z = 0;
+            Tr::run_segment(sv, n, seg, segs, seg_smem, S, t, d);
+            if (threadIdx.x == 0) S.pend = 0;
+            if (seg.stats) {
+              Tr::block_sum3(S, t, d, z);
+              T = t;
+              Dd = d;
+            } else {
+              __syncthreads();
+            }
+            stats_valid = seg.stats != 0;
+            ev += seg.n_err;
+            oi = seg.end_op - 1;
+            continue;
+          }
+        }
+      }
       if (op.type == T_GATE) {
         if (op.stats) Tr::fill_stab(S, (double)op.sgamma);
         Tr::stage_matrix(Msm, pool, op.mat, 1u << (2 * op.k));
@@ -582,7 +809,9 @@ constexpr uint32_t kTrajMagic = 0xCB2077A1u;
 // Threads per CTA when the program does not fix them: 1024 for states of 15 to
 // 17 qubits (slices larger than L1 but held in L2, so passes are bound by loads
 // in flight), 512 otherwise (issue-bound gate arithmetic).
-unsigned auto_threads(uint32_t n) { return n >= 15 && n <= 17 ? 1024u : 512u; }
+// A program with merged segments takes 512 for every size: their passes hold tiles
+// in shared memory, and their gate code needs the registers.
+unsigned auto_threads(uint32_t n, bool segments) { return !segments && n >= 15 && n <= 17 ? 1024u : 512u; }
 
 // Trajectories in flight when the program does not fix them: one per SM, unless
 // the slices of one per SM overflow L2 while those of at least half as many
@@ -607,15 +836,23 @@ unsigned auto_ctas(uint32_t n) {
 // 2.8 TB/s until it was set back to 0.
 cudaError_t launch_trajectories(unsigned grid, unsigned threads, cudaStream_t s, const TOp *ops,
                                 uint32_t n_ops, const float2 *pool, float2 *ws, uint32_t n,
-                                const TRun *run, double *z, uint32_t *sample) {
+                                const TRun *run, double *z, uint32_t *sample, TSegs segs) {
+  if (threads != (unsigned)kTMinThreads) segs.segs = nullptr;  // segments need 128 registers a thread
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes =
+      segs.segs ? segs.mat_cap + kSegArgBytes + (sizeof(float2) << (1 + std::min(n, kSegMaxTile))) : 0;
+  if (cfg.dynamicSmemBytes) {
+    const cudaError_t rc = cudaFuncSetAttribute(k_trajectories<kTMinThreads>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)cfg.dynamicSmemBytes);
+    if (rc != cudaSuccess) return rc;
+  }
   cfg.stream = s;
   if (threads == 1024)
-    return cudaLaunchKernelEx(&cfg, k_trajectories<1024>, ops, n_ops, pool, ws, n, run, z, sample);
-  return cudaLaunchKernelEx(&cfg, k_trajectories<512>, ops, n_ops, pool, ws, n, run, z, sample);
+    return cudaLaunchKernelEx(&cfg, k_trajectories<1024>, ops, n_ops, pool, ws, n, run, z, sample, segs);
+  return cudaLaunchKernelEx(&cfg, k_trajectories<512>, ops, n_ops, pool, ws, n, run, z, sample, segs);
 }
 
 // Device buffers of trajectory programs come from a process-wide cache keyed by
@@ -673,6 +910,9 @@ struct TrajProgram {
   float2 *d_ws = nullptr;
   size_t ws_ctas = 0;
   size_t ops_bytes = 0, pool_bytes = 0, ws_bytes = 0, z_bytes = 0, sample_bytes = 0;
+  void *d_segs = nullptr;     // the segments' arrays, one buffer
+  size_t segs_bytes = 0;
+  TSegs segs{};
   TRun *d_run = nullptr;
   double *d_z = nullptr;
   uint32_t *d_sample = nullptr;
@@ -690,6 +930,7 @@ struct TrajProgram {
     buf_free(d_ops, ops_bytes);
     buf_free(d_pool, pool_bytes);
     buf_free(d_ws, ws_bytes);
+    buf_free(d_segs, segs_bytes);
     buf_free(d_run, sizeof(TRun));
     buf_free(d_z, z_bytes);
     buf_free(d_sample, sample_bytes);
@@ -721,9 +962,119 @@ struct TrajProgram {
     }
   }
 
+  // Groups every run of GATE ops into passes and uploads the segments that come out
+  // with fewer passes than gates.
+  bool build_segments(std::string &err) {
+    std::vector<TSeg> sg;
+    std::vector<TSegPass> ps;
+    std::vector<cb2::PassGateArgs32> gs;
+    std::vector<uint32_t> sites;
+    std::vector<float> mats;
+    uint32_t mat_cap = 0;
+    const uint32_t tb_most = std::min(n, kSegMaxTile);
+    for (auto &o : ops) o.seg = 0;
+    for (size_t i = 0; i < ops.size() && n >= kSegMinQubits; ++i) {
+      if (ops[i].type != T_GATE) continue;
+      size_t end = i;
+      std::vector<cb2::GateData> gates;
+      TSeg g{};
+      g.err0 = (uint32_t)sites.size();
+      for (; end < ops.size() && (ops[end].type == T_GATE || ops[end].type == T_ERR); ++end) {
+        if (ops[end].type == T_ERR) {
+          sites.push_back((uint32_t)end);
+          continue;
+        }
+        cb2::GateData x;
+        x.k = ops[end].k;
+        for (uint32_t b = 0; b < x.k; ++b) x.qubits[b] = ops[end].q[b];
+        const size_t entries = size_t(1) << (2 * x.k);
+        x.m64.reserve(2 * entries);
+        for (size_t e = 0; e < entries; ++e) {
+          x.m64.push_back(pool[ops[end].mat + e].x);
+          x.m64.push_back(pool[ops[end].mat + e].y);
+        }
+        if (ops[end].stats) {
+          g.stats = 1;
+          g.smask = ops[end].smask;
+          g.sgamma = ops[end].sgamma;
+        }
+        gates.push_back(std::move(x));
+      }
+      g.n_err = (uint32_t)sites.size() - g.err0;
+      g.end_op = (uint32_t)end;
+      std::vector<cb2::PassGate> pg(gates.size());
+      for (size_t j = 0; j < gates.size(); ++j) {
+        for (uint32_t b = 0; b < gates[j].k; ++b) pg[j].qubits |= 1ull << gates[j].qubits[b];
+        pg[j].mergeable = true;
+      }
+      const std::vector<cb2::Pass> passes =
+          cb2::plan_passes(pg, n, tb_most, kSegLow, cb2::kMaxPassGates, 11);
+      if (passes.size() >= gates.size()) {
+        sites.resize(g.err0);
+        i = end - 1;
+        continue;
+      }
+      g.pass0 = (uint32_t)ps.size();
+      g.n_passes = (uint32_t)passes.size();
+      for (const cb2::Pass &x : passes) {
+        uint64_t tile = x.tile ? x.tile : pg[x.gates[0]].qubits | ((1ull << std::min(n, kSegLow)) - 1);
+        for (uint32_t b = 0; b < n && (uint32_t)__builtin_popcountll(tile) < tb_most; ++b) tile |= 1ull << b;
+        std::vector<uint32_t> qubits;
+        for (uint32_t q = 0; q < n; ++q)
+          if ((tile >> q) & 1) qubits.push_back(q);
+        TSegPass t{};
+        t.tb = (uint32_t)qubits.size();
+        t.n_gates = (uint32_t)x.gates.size();
+        t.gate0 = (uint32_t)gs.size();
+        t.mat = (uint32_t)mats.size();
+        for (uint32_t j = 0; j < t.tb; ++j) t.stride[j] = 1u << qubits[j];
+        for (const uint32_t j : x.gates) {
+          cb2::PassGateArgs32 a;
+          cb2::pack_gate32(cb2::place_gate(gates[j], qubits, 2), t.tb, false, mats, a);
+          gs.push_back(a);
+        }
+        t.mat_bytes = (uint32_t)((mats.size() - t.mat) * sizeof(float));
+        mat_cap = std::max(mat_cap, t.mat_bytes);
+        ps.push_back(t);
+      }
+      ops[i].seg = (uint32_t)sg.size() + 1;
+      sg.push_back(g);
+      i = end - 1;
+    }
+    buf_free(d_segs, segs_bytes);
+    d_segs = nullptr;
+    segs_bytes = 0;
+    segs = TSegs{};
+    if (sg.empty()) return true;
+    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t at_p = align(sg.size() * sizeof(TSeg)), at_g = at_p + align(ps.size() * sizeof(TSegPass)),
+                 at_s = at_g + align(gs.size() * sizeof(gs[0])), at_m = at_s + align(sites.size() * 4 + 4),
+                 bytes = at_m + align(mats.size() * sizeof(float));
+    std::vector<char> host(bytes, 0);
+    std::memcpy(host.data(), sg.data(), sg.size() * sizeof(TSeg));
+    std::memcpy(host.data() + at_p, ps.data(), ps.size() * sizeof(TSegPass));
+    std::memcpy(host.data() + at_g, gs.data(), gs.size() * sizeof(gs[0]));
+    std::memcpy(host.data() + at_s, sites.data(), sites.size() * 4);
+    std::memcpy(host.data() + at_m, mats.data(), mats.size() * sizeof(float));
+    if (!cuda_ok(buf_alloc(&d_segs, bytes), "cudaMalloc (trajectory segments)", err)) return false;
+    segs_bytes = bytes;
+    if (!cuda_ok(cudaMemcpy(d_segs, host.data(), bytes, cudaMemcpyHostToDevice),
+                 "cudaMemcpy (trajectory segments)", err))
+      return false;
+    const char *base = static_cast<const char *>(d_segs);
+    segs.segs = reinterpret_cast<const TSeg *>(base);
+    segs.passes = reinterpret_cast<const TSegPass *>(base + at_p);
+    segs.gates = reinterpret_cast<const cb2::PassGateArgs32 *>(base + at_g);
+    segs.sites = reinterpret_cast<const uint32_t *>(base + at_s);
+    segs.mats = reinterpret_cast<const float *>(base + at_m);
+    segs.mat_cap = (mat_cap + 15) & ~15u;
+    return true;
+  }
+
   bool upload(std::string &err) {
     if (!dirty) return true;
     mark_stats();
+    if (!build_segments(err)) return false;
     if (graph) {
       cudaGraphExecDestroy(graph);
       graph = nullptr;
@@ -972,7 +1323,7 @@ int cast_b200_traj_run_range(void *prog, uint32_t first, uint32_t n_traj, uint64
     }
     const unsigned ctas = p->max_ctas ? p->max_ctas : auto_ctas(p->n);
     const unsigned grid = (unsigned)std::min<uint64_t>(n_traj, ctas);
-    const unsigned threads = p->threads ? p->threads : auto_threads(p->n);
+    const unsigned threads = p->threads ? p->threads : auto_threads(p->n, p->segs.segs != nullptr);
     if (p->ws_ctas < grid) {
       buf_free(p->d_ws, p->ws_bytes);
       p->d_ws = nullptr;
@@ -1038,7 +1389,7 @@ int cast_b200_traj_run_range(void *prog, uint32_t first, uint32_t n_traj, uint64
           return 1;
         }
         const cudaError_t lrc = launch_trajectories(grid, threads, s, p->d_ops, n_ops, p->d_pool,
-                                                    p->d_ws, p->n, p->d_run, p->d_z, p->d_sample);
+                                                    p->d_ws, p->n, p->d_run, p->d_z, p->d_sample, p->segs);
         const cudaError_t erc = cudaStreamEndCapture(s, &gph);
         if (!cuda_ok(lrc, "trajectory kernel capture", err) ||
             !cuda_ok(erc, "cudaStreamEndCapture", err) ||
@@ -1058,7 +1409,7 @@ int cast_b200_traj_run_range(void *prog, uint32_t first, uint32_t n_traj, uint64
       }
     } else {
       if (!cuda_ok(launch_trajectories(grid, threads, s, p->d_ops, n_ops, p->d_pool, p->d_ws, p->n,
-                                       p->d_run, p->d_z, p->d_sample),
+                                       p->d_run, p->d_z, p->d_sample, p->segs),
                    "trajectory kernel launch", err)) {
         cb2::write_err(err_buf, err_buf_len, err);
         return 1;
