@@ -643,17 +643,18 @@ bool scale_popc_impl(void *x, uint32_t n, uint64_t mask, double sfac, double sca
 
 template <typename T>
 bool dm_impl(const void *rho, uint32_t n, double *out, cudaStream_t s, std::string &err) {
-  double *d = nullptr;
-  const size_t bytes = sizeof(double) << n;
-  if (!cuda_ok(cudaMallocAsync(&d, bytes, s), "cudaMallocAsync (dm diagonal)", err)) return false;
+  // into the reductions' scratch: a stream-ordered allocation here is handed back at
+  // the synchronise and mapped again by the next call
+  std::lock_guard<std::mutex> lock(g_scratch_mu);
   const uint64_t dim = 1ull << n;
+  Scratch *const sc = ensure_scratch((int)dim, err);
+  if (!sc) return false;
   const unsigned grid = (unsigned)std::min<uint64_t>((dim + 255) / 256, 4ull * sm_count());
-  k_dm_diag<T><<<grid, 256, 0, s>>>(static_cast<const T *>(rho), n, d);
-  const bool ok = cuda_ok(cudaGetLastError(), "dm diagonal launch", err) &&
-                  cuda_ok(cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, s),
-                          "cudaMemcpyAsync (dm diagonal)", err);
-  cudaFreeAsync(d, s);
-  return ok && cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (dm diagonal)", err);
+  k_dm_diag<T><<<grid, 256, 0, s>>>(static_cast<const T *>(rho), n, sc->partial);
+  return cuda_ok(cudaGetLastError(), "dm diagonal launch", err) &&
+         cuda_ok(cudaMemcpyAsync(out, sc->partial, sizeof(double) << n, cudaMemcpyDeviceToHost, s),
+                 "cudaMemcpyAsync (dm diagonal)", err) &&
+         cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (dm diagonal)", err);
 }
 
 }  // namespace
