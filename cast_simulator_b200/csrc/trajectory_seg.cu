@@ -13,6 +13,16 @@ __global__ void __launch_bounds__(kTMinThreads, 1)
   trajectories<kTMinThreads, true>(ops, n_ops, pool, ws, n, run, out_z, out_sample, segs, seg_smem);
 }
 
+// Shared memory of the largest launch: a full pass of 4-qubit gates and two tiles of
+// the largest size.  The limit is the kernel's, shared by every program of the
+// process: set to what one program needs, it would fall under the launch of another
+// that a second thread is making.
+constexpr size_t kSegSmemMost =
+    cb2::kMaxPassGates * cb2::kPass32MatBytes + kSegArgBytes + (sizeof(float2) << (1 + kSegMaxTile));
+static_assert(kSegSmemMost + sizeof(Shared) + (sizeof(float2) << (2 * kTrajMaxGate)) +
+                      sizeof(double) * kTMinThreads <= 227 * 1024,
+              "fits a CTA beside the static arrays");
+
 }  // namespace
 
 namespace cb2 {
@@ -23,7 +33,7 @@ cudaError_t launch_trajectory_segments(unsigned grid, cudaStream_t s, const void
   const TSegs &g = *static_cast<const TSegs *>(segs);
   const size_t smem = g.mat_cap + kSegArgBytes + (sizeof(float2) << (1 + std::min(n, kSegMaxTile)));
   const cudaError_t rc =
-      cudaFuncSetAttribute(k_trajectories_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(k_trajectories_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSegSmemMost);
   if (rc != cudaSuccess) return rc;
   k_trajectories_seg<<<grid, kTMinThreads, smem, s>>>(static_cast<const TOp *>(ops), n_ops, pool, ws, n,
                                                       static_cast<const TRun *>(run), z, sample, g);
