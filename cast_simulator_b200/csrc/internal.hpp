@@ -28,9 +28,12 @@ struct GateData {
   void *d_sparse = nullptr;  // CSR copy for the sparse kernel (owned by the holder), if any
 };
 
-// Error helper: fills `err` and returns false on a CUDA failure.
+// Error helper: fills `err` and returns false on a CUDA failure.  What is reported
+// here is taken out of the runtime's per-thread last error, where the status check
+// behind the thread's next launch would find it and call that launch failed.
 inline bool cuda_ok(cudaError_t rc, const char *what, std::string &err) {
   if (rc == cudaSuccess) return true;
+  cudaGetLastError();
   err = std::string(what) + " failed: " + cudaGetErrorName(rc) + " - " + cudaGetErrorString(rc);
   return false;
 }

@@ -35,9 +35,13 @@ cudaError_t launch_trajectory_segments(unsigned grid, cudaStream_t s, const void
   const cudaError_t rc =
       cudaFuncSetAttribute(k_trajectories_seg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSegSmemMost);
   if (rc != cudaSuccess) return rc;
-  k_trajectories_seg<<<grid, kTMinThreads, smem, s>>>(static_cast<const TOp *>(ops), n_ops, pool, ws, n,
-                                                      static_cast<const TRun *>(run), z, sample, g);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kTMinThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, k_trajectories_seg, static_cast<const TOp *>(ops), n_ops, pool, ws, n,
+                            static_cast<const TRun *>(run), z, sample, g);
 }
 
 }  // namespace cb2

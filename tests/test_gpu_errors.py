@@ -1,0 +1,57 @@
+"""Calls that follow a refused one: its status never becomes that of a later launch."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _brickwork(n, seed, **noise):
+    from cast_simulator_b200.types import QuantumCircuit
+
+    return QuantumCircuit.brickwork(n, 4, seed, **noise)
+
+
+def _refused(cblib):
+    """A device allocation that no GPU can give (16 TiB)."""
+    from cast_simulator_b200.cuda import CudaPrecision, CudaStatevector
+
+    with pytest.raises(RuntimeError):
+        CudaStatevector(40, CudaPrecision.F64)
+
+
+@pytest.mark.parametrize("call", ["norm", "populations", "marginal", "overlap", "program", "batch",
+                                  "sample", "trajectories"])
+def test_a_refused_allocation_leaves_later_calls_alone(cblib, call):
+    from cast_simulator_b200 import simulator as S
+    from cast_simulator_b200.cuda import CudaPrecision, CudaStatevector
+    from cast_simulator_b200.trajectory import TrajectoryProgram
+
+    n, st = 10, S.Stream()
+    sv = CudaStatevector(n, CudaPrecision.F64)
+    sv.zero()
+    gates = _brickwork(n, 3).gates()
+    prog, batch = S.GateProgram(CudaPrecision.F64, n, 1e-12, 1e-12), S.CircuitBatch()
+    for g in gates:
+        prog.add(g.matrix(), g.qubits())
+    batch.add(sv, gates)
+    traj = TrajectoryProgram(_brickwork(n, 3, depolarizing=1e-3), 3)
+    want = traj.run(3, 5)[0]
+    _refused(cblib)
+    if call == "norm":
+        assert abs(sv.norm_squared() - 1) < 1e-12
+    elif call == "populations":
+        assert np.allclose(S.qubit_populations(sv, st)[0], 0)
+    elif call == "marginal":
+        assert np.allclose(S.marginal_probabilities(sv, [1, 4], st), [1, 0, 0, 0])
+    elif call == "overlap":
+        assert abs(S.inner_product(sv, sv, st) - 1) < 1e-12
+    elif call == "program":
+        prog.run(sv, st)
+        st.sync()
+        assert abs(sv.norm_squared() - 1) < 1e-12
+    elif call == "batch":
+        assert len(batch.run(st)[0]) == n
+    elif call == "sample":
+        assert (S.sample(sv, 16, 1, stream=st) == 0).all()
+    else:
+        assert np.array_equal(traj.run(3, 5, st)[0], want)
