@@ -48,19 +48,16 @@ template <typename T> struct V16;
 template <> struct V16<float> { using type = float4; static constexpr int N = 4; };
 template <> struct V16<double> { using type = double2; static constexpr int N = 2; };
 
-// Blocks of the running launch that have written their partials.  One reduction
-// runs at a time (the scratch mutex) and its last block puts the count back to 0.
-__device__ unsigned g_blocks_done;
-
 // Called by every block once its partials are written: true in the block that
-// comes last, for which all partials are then visible.
-__device__ __forceinline__ bool last_block() {
+// comes last, for which all partials are then visible.  `done` counts the blocks of
+// the running launch; the last one puts it back to 0.
+__device__ __forceinline__ bool last_block(unsigned *done) {
   __shared__ bool last;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    last = atomicAdd(&g_blocks_done, 1u) == gridDim.x - 1;
-    if (last) g_blocks_done = 0;
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+    if (last) *done = 0;
   }
   __syncthreads();
   if (last) __threadfence();
@@ -90,7 +87,8 @@ __device__ __forceinline__ void fold_columns(const double *partial, int rows, in
 
 // out[0] = sum of squares.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_norm(const T *__restrict__ x, uint64_t n, double *partial,
+__global__ void __launch_bounds__(kRedThreads) k_norm(const T *__restrict__ x, uint64_t n,
+                                                     double *partial, unsigned *done,
                                                      double *__restrict__ out) {
   using V = typename V16<T>::type;
   constexpr int N = V16<T>::N;
@@ -115,7 +113,7 @@ __global__ void __launch_bounds__(kRedThreads) k_norm(const T *__restrict__ x, u
   }
   acc = block_sum(acc);
   if (threadIdx.x == 0) partial[blockIdx.x] = acc;
-  if (last_block()) fold_columns(partial, (int)gridDim.x, 1, out);
+  if (last_block(done)) fold_columns(partial, (int)gridDim.x, 1, out);
 }
 
 template <typename T>
@@ -137,21 +135,23 @@ __global__ void __launch_bounds__(kRedThreads) k_scale(T *__restrict__ x, uint64
   if (blockIdx.x == 0 && threadIdx.x < n - nv * N) x[nv * N + threadIdx.x] *= s;
 }
 
-// Scratch of one device: per-block partials and a page-locked result buffer that
-// kernels write straight into.  Allocated on first use and grown on demand (the reference
-// keeps the same kind of process-wide scratch, cuda_kernels.cu:203-230).  The
-// mutex serialises its users, each until its result has arrived.
+// Scratch of one device: per-block partials, the count of finished blocks and a
+// page-locked result buffer that kernels write straight into.  Allocated on first use
+// and grown on demand (the reference keeps the same kind of process-wide scratch,
+// cuda_kernels.cu:203-230).  The mutex serialises its users, each until its result
+// has arrived.
 std::mutex g_scratch_mu;
 constexpr int kMaxScratchDevices = 64;
 constexpr int kMaxResult = 4096;  // doubles: the largest marginal
 struct Scratch {
   double *partial = nullptr;
   int len = 0;
+  unsigned *done = nullptr;  // 0 between launches
   double *result = nullptr;  // page-locked, mapped
 };
 Scratch g_scratch_dev[kMaxScratchDevices];
 
-Scratch *ensure_scratch(int len, std::string &err) {
+Scratch *ensure_scratch(int len, cudaStream_t stream, std::string &err) {
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return nullptr;
   if (dev < 0 || dev >= kMaxScratchDevices) {
@@ -165,21 +165,38 @@ Scratch *ensure_scratch(int len, std::string &err) {
     s.result = nullptr;
     return nullptr;
   }
-  if (s.partial && s.len >= len) return &s;
-  if (s.partial) cudaFree(s.partial);
-  s.partial = nullptr;
-  s.len = 0;
-  if (!cuda_ok(cudaMalloc((void **)&s.partial, sizeof(double) * len), "cudaMalloc (norm scratch)", err)) {
+  if (!s.partial || s.len < len) {
+    if (s.partial) cudaFree(s.partial);
     s.partial = nullptr;
-    return nullptr;
+    s.len = 0;
+    if (!cuda_ok(cudaMalloc((void **)&s.partial, sizeof(double) * len), "cudaMalloc (norm scratch)", err)) {
+      s.partial = nullptr;
+      return nullptr;
+    }
+    s.len = len;
   }
-  s.len = len;
+  if (!s.done) {
+    unsigned *done = nullptr;
+    if (!cuda_ok(cudaMalloc((void **)&done, sizeof(unsigned)), "cudaMalloc (reduction count)", err)) return nullptr;
+    // ahead of the caller's launch on this stream, which it waits for
+    if (!cuda_ok(cudaMemsetAsync(done, 0, sizeof(unsigned), stream), "cudaMemsetAsync (reduction count)", err)) {
+      cudaFree(done);
+      return nullptr;
+    }
+    s.done = done;
+  }
   return &s;
 }
 
-// Launch status, then the wait for the result in s.result.
-bool fetch_result(cudaStream_t stream, const char *what, std::string &err) {
-  return cuda_ok(cudaGetLastError(), what, err) && cuda_ok(cudaStreamSynchronize(stream), what, err);
+// Launch status and the wait for the result in s.result: always both, since a kernel
+// still running would go on using the scratch after the mutex is free.  Where the
+// wait itself fails nothing says that the kernel has ended or what it leaves in the
+// count: the scratch is given up (not freed) and the next reduction makes its own.
+bool fetch_result(Scratch &s, cudaStream_t stream, const char *what, std::string &err) {
+  const cudaError_t launched = cudaGetLastError();
+  const cudaError_t waited = cudaStreamSynchronize(stream);
+  if (waited != cudaSuccess) s = Scratch{};
+  return cuda_ok(launched, what, err) && cuda_ok(waited, what, err);
 }
 
 unsigned red_grid(uint64_t nv) {
@@ -192,10 +209,11 @@ template <typename T>
 bool norm_sq_impl(const void *x, uint64_t n, double *out, cudaStream_t s, std::string &err) {
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   const unsigned grid = red_grid(n / V16<T>::N);
-  Scratch *const sc = ensure_scratch((int)grid, err);
+  Scratch *const sc = ensure_scratch((int)grid, s, err);
   if (!sc) return false;
-  k_norm<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->partial, sc->result);
-  if (!fetch_result(s, "norm", err)) return false;
+  k_norm<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->partial, sc->done,
+                                         sc->result);
+  if (!fetch_result(*sc, s, "norm", err)) return false;
   *out = sc->result[0];
   return true;
 }
@@ -225,7 +243,7 @@ __device__ __forceinline__ void inner_add(double2 x, double2 y, double &re, doub
 // states, 0.60 of the copy peak; now 356 us).
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_inner(const T *__restrict__ a, const T *__restrict__ b,
-                                                      uint64_t n_vec, double *partial,
+                                                      uint64_t n_vec, double *partial, unsigned *done,
                                                       double *__restrict__ out) {
   using V = typename V16<T>::type;
   const V *av = reinterpret_cast<const V *>(a);
@@ -255,7 +273,7 @@ __global__ void __launch_bounds__(kRedThreads) k_inner(const T *__restrict__ a, 
     partial[2 * blockIdx.x] = r;
     partial[2 * blockIdx.x + 1] = m;
   }
-  if (last_block()) fold_columns(partial, (int)gridDim.x, 2, out);
+  if (last_block(done)) fold_columns(partial, (int)gridDim.x, 2, out);
 }
 
 constexpr int kMaxPopQubits = 40;
@@ -282,7 +300,8 @@ constexpr uint32_t kPopRowBits = 3;  // rows a thread takes at once, all loads i
 // neighbour's).
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, 2) k_populations(const T *__restrict__ x, uint32_t n,
-                                                               double *partial, double *__restrict__ out) {
+                                                               double *partial, unsigned *done,
+                                                               double *__restrict__ out) {
   using V = typename V16<T>::type;
   constexpr uint32_t VB = vec_bits<T>(), CB = row_bits<T>() + kPopRowBits;
   constexpr int R = 1 << kPopRowBits;
@@ -336,7 +355,7 @@ __global__ void __launch_bounds__(kRedThreads, 2) k_populations(const T *__restr
   for (uint32_t q = 0; q < kMaxPopQubits - CB; ++q)
     if (CB + q < n) put(CB + q, high[q]);
   put(n, tot);
-  if (last_block()) fold_columns(partial, (int)gridDim.x, (int)n + 1, out);
+  if (last_block(done)) fold_columns(partial, (int)gridDim.x, (int)n + 1, out);
 }
 
 // The same for a state below one chunk: one block, amplitude by amplitude.
@@ -475,7 +494,8 @@ struct PopcTable {
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads) k_damp_sums(const T *__restrict__ x, uint32_t n,
                                                           uint64_t mask, const PopcTable tab,
-                                                          double *partial, double *__restrict__ out) {
+                                                          double *partial, unsigned *done,
+                                                          double *__restrict__ out) {
   using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
   const V *xv = reinterpret_cast<const V *>(x);
   const uint64_t n_amps = 1ull << n;
@@ -494,7 +514,7 @@ __global__ void __launch_bounds__(kRedThreads) k_damp_sums(const T *__restrict__
     partial[2 * blockIdx.x] = t;
     partial[2 * blockIdx.x + 1] = d;
   }
-  if (last_block()) fold_columns(partial, (int)gridDim.x, 2, out);
+  if (last_block(done)) fold_columns(partial, (int)gridDim.x, 2, out);
 }
 
 // x_i *= scale * s^popc(i & mask): the no-jump branch of amplitude damping on
@@ -530,11 +550,11 @@ bool inner_impl(const void *a, const void *b, uint32_t n, double *re, double *im
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   const uint64_t vec = (1ull << n) >> vec_bits<T>();
   const unsigned grid = red_grid(vec);
-  Scratch *const sc = ensure_scratch(2 * (int)grid, err);
+  Scratch *const sc = ensure_scratch(2 * (int)grid, s, err);
   if (!sc) return false;
   k_inner<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(a), static_cast<const T *>(b), vec,
-                                          sc->partial, sc->result);
-  if (!fetch_result(s, "inner product", err)) return false;
+                                          sc->partial, sc->done, sc->result);
+  if (!fetch_result(*sc, s, "inner product", err)) return false;
   *re = sc->result[0];
   *im = sc->result[1];
   return true;
@@ -547,13 +567,14 @@ bool pop_impl(const void *x, uint32_t n, double *p1, double *norm, cudaStream_t 
   constexpr uint32_t CB = row_bits<T>() + kPopRowBits;
   const uint64_t chunks = n >= CB ? 1ull << (n - CB) : 1;
   const unsigned grid = (unsigned)std::min<uint64_t>(chunks, 2ull * sm_count());
-  Scratch *const sc = ensure_scratch((int)((n + 1) * grid), err);
+  Scratch *const sc = ensure_scratch((int)((n + 1) * grid), s, err);
   if (!sc) return false;
   if (n >= CB)
-    k_populations<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->partial, sc->result);
+    k_populations<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->partial, sc->done,
+                                                  sc->result);
   else
     k_populations_small<T><<<1, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, sc->result);
-  if (!fetch_result(s, "populations", err)) return false;
+  if (!fetch_result(*sc, s, "populations", err)) return false;
   for (uint32_t q = 0; q < n; ++q) p1[q] = sc->result[q];
   if (norm) *norm = sc->result[n];
   return true;
@@ -582,12 +603,12 @@ bool marg_impl(const void *x, uint32_t n, const uint32_t *measured, uint32_t m, 
   const uint32_t bins = 1u << (a.high_bits + a.in_bits);
   const unsigned grid = 1u << (a.high_bits + a.segs_log2);
   std::lock_guard<std::mutex> lock(g_scratch_mu);
-  Scratch *const sc = ensure_scratch((int)(grid << a.in_bits), err);
+  Scratch *const sc = ensure_scratch((int)(grid << a.in_bits), s, err);
   if (!sc) return false;
   k_marginal_rows<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, a, sc->partial);
   k_marginal_fold<<<std::min<uint32_t>((bins + 7) / 8, 512), kRedThreads, 0, s>>>(
       sc->partial, bins, a.in_bits, a.segs_log2, sc->result);
-  if (!fetch_result(s, "marginal", err)) return false;
+  if (!fetch_result(*sc, s, "marginal", err)) return false;
   // out[i]: the bin whose bits are i's at the measured qubits' places
   uint32_t bin[1u << 12], place[12];
   bool listed_once = true;
@@ -623,11 +644,11 @@ bool damp_sums_impl(const void *x, uint32_t n, uint64_t mask, double gamma, doub
                     cudaStream_t s, std::string &err) {
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   const unsigned grid = red_grid(1ull << n);
-  Scratch *const sc = ensure_scratch(2 * (int)grid, err);
+  Scratch *const sc = ensure_scratch(2 * (int)grid, s, err);
   if (!sc) return false;
   k_damp_sums<T><<<grid, kRedThreads, 0, s>>>(static_cast<const T *>(x), n, mask, powers(1.0 - gamma, 1.0),
-                                              sc->partial, sc->result);
-  if (!fetch_result(s, "damping sums", err)) return false;
+                                              sc->partial, sc->done, sc->result);
+  if (!fetch_result(*sc, s, "damping sums", err)) return false;
   *tot = sc->result[0];
   *wsum = sc->result[1];
   return true;
@@ -647,14 +668,15 @@ bool dm_impl(const void *rho, uint32_t n, double *out, cudaStream_t s, std::stri
   // the synchronise and mapped again by the next call
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   const uint64_t dim = 1ull << n;
-  Scratch *const sc = ensure_scratch((int)dim, err);
+  Scratch *const sc = ensure_scratch((int)dim, s, err);
   if (!sc) return false;
   const unsigned grid = (unsigned)std::min<uint64_t>((dim + 255) / 256, 4ull * sm_count());
   k_dm_diag<T><<<grid, 256, 0, s>>>(static_cast<const T *>(rho), n, sc->partial);
-  return cuda_ok(cudaGetLastError(), "dm diagonal launch", err) &&
-         cuda_ok(cudaMemcpyAsync(out, sc->partial, sizeof(double) << n, cudaMemcpyDeviceToHost, s),
-                 "cudaMemcpyAsync (dm diagonal)", err) &&
-         cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (dm diagonal)", err);
+  const bool copied =
+      cuda_ok(cudaGetLastError(), "dm diagonal launch", err) &&
+      cuda_ok(cudaMemcpyAsync(out, sc->partial, sizeof(double) << n, cudaMemcpyDeviceToHost, s),
+              "cudaMemcpyAsync (dm diagonal)", err);
+  return fetch_result(*sc, s, "dm diagonal", err) && copied;
 }
 
 }  // namespace

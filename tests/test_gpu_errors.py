@@ -55,3 +55,36 @@ def test_a_refused_allocation_leaves_later_calls_alone(cblib, call):
         assert (S.sample(sv, 16, 1, stream=st) == 0).all()
     else:
         assert np.array_equal(traj.run(3, 5, st)[0], want)
+
+
+def test_reductions_on_many_streams_between_refusals(cblib):
+    """Threads share one scratch and one count of finished blocks: every result stays
+    that of its own state while other threads' allocations are refused."""
+    import threading
+
+    from cast_simulator_b200 import simulator as S
+    from cast_simulator_b200.cuda import CudaPrecision, CudaStatevector
+
+    wrong = []
+
+    def work(j):
+        n, st = 12 + 3 * j, S.Stream()
+        sv = CudaStatevector(n, CudaPrecision.F64 if j % 2 else CudaPrecision.F32)
+        sv.zero()
+        try:
+            for i in range(30):
+                if i % 5 == j % 5:
+                    _refused(cblib)
+                p, norm = S.qubit_populations(sv, st)
+                m = S.marginal_probabilities(sv, [0, n - 1], st)
+                if norm != 1 or p.any() or m.tolist() != [1, 0, 0, 0] or S.inner_product(sv, sv, st) != 1:
+                    wrong.append((j, i))
+        except Exception as e:
+            wrong.append((j, str(e)))
+
+    threads = [threading.Thread(target=work, args=(j,)) for j in range(5)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:4]
