@@ -22,6 +22,7 @@
 // once 291, larger MMA shapes (m16n8k8, m16n8k16) 294.
 #include "gate_tile.cuh"
 #include "pass_plan.hpp"
+#include "plan_buffers.hpp"
 
 #include <memory>
 #include <mutex>
@@ -171,77 +172,26 @@ __global__ void __launch_bounds__(kPassThreads, 3)
 
 // ── host side ────────────────────────────────────────────────────────────────
 
-// Device buffers of plans.  A plan's buffer may still be read by launches in
-// flight when its program is destroyed, so it comes back with the events recorded
-// behind those launches and is handed out again (or freed) only once they have
-// completed.  At most kPoolBytes wait here; a buffer beyond that is freed, which
-// waits for the device.
-constexpr size_t kPoolBytes = size_t(64) << 20;
-
-struct PoolBuffer {
-  int device = 0;
-  char *ptr = nullptr;
-  size_t bytes = 0;
-  std::vector<cudaEvent_t> events;
+// The runtime calls behind plan_buffers.hpp; a call that fails says why in `err`.
+struct PlanApi {
+  using Event = cudaEvent_t;
+  using Stream = cudaStream_t;
+  std::string &err;
+  bool done(Event e) { return cudaEventQuery(e) == cudaSuccess; }
+  bool record(Event e, Stream s) { return cuda_ok(cudaEventRecord(e, s), "cudaEventRecord (gate pass)", err); }
+  bool create(Event &e) {
+    return cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate (gate pass)", err);
+  }
+  void destroy(Event e) { cudaEventDestroy(e); }
+  bool allocate(size_t bytes, char *&p) {
+    return cuda_ok(cudaMalloc((void **)&p, bytes), "cudaMalloc (gate pass matrices)", err);
+  }
+  void release(char *p) { cudaFree(p); }
 };
 
-struct BufferPool {
-  std::mutex mu;
-  std::vector<PoolBuffer> idle;
-  size_t total = 0;
-};
-
-BufferPool &buffer_pool() {
-  static BufferPool *p = new BufferPool;  // outlives programs destroyed at exit
+PlanBufferPool<PlanApi> &buffer_pool() {
+  static auto *p = new PlanBufferPool<PlanApi>(size_t(64) << 20);  // outlives programs destroyed at exit
   return *p;
-}
-
-bool settled(PoolBuffer &b) {
-  while (!b.events.empty()) {
-    if (cudaEventQuery(b.events.back()) == cudaErrorNotReady) return false;
-    cudaEventDestroy(b.events.back());
-    b.events.pop_back();
-  }
-  return true;
-}
-
-bool take_buffer(size_t bytes, PoolBuffer &out, std::string &err) {
-  size_t cap = size_t(64) << 10;
-  while (cap < bytes) cap <<= 1;
-  int dev = 0;
-  if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return false;
-  {
-    BufferPool &p = buffer_pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    for (size_t i = 0; i < p.idle.size(); ++i)
-      if (p.idle[i].device == dev && p.idle[i].bytes == cap && settled(p.idle[i])) {
-        out = p.idle[i];
-        p.total -= cap;
-        p.idle.erase(p.idle.begin() + (std::ptrdiff_t)i);
-        return true;
-      }
-  }
-  out = PoolBuffer{};
-  out.device = dev;
-  out.bytes = cap;
-  return cuda_ok(cudaMalloc((void **)&out.ptr, cap), "cudaMalloc (gate pass matrices)", err);
-}
-
-void give_buffer(PoolBuffer &b) {
-  if (!b.ptr) return;
-  {
-    BufferPool &p = buffer_pool();
-    std::lock_guard<std::mutex> lock(p.mu);
-    if (p.total + b.bytes <= kPoolBytes) {
-      p.total += b.bytes;
-      p.idle.push_back(std::move(b));
-      b = PoolBuffer{};
-      return;
-    }
-  }
-  cudaFree(b.ptr);  // waits for the device
-  for (cudaEvent_t e : b.events) cudaEventDestroy(e);
-  b = PoolBuffer{};
 }
 
 // Copies `bytes` to the device on a stream of its own and waits for that copy
@@ -282,8 +232,7 @@ struct PassPlan {
   std::vector<int> arg_of;      // pass -> its entry of args, -1 for a single gate
   std::vector<double> pool;     // matrices of every merged gate, as its kernel reads them
   std::vector<float> pool32;    // the same in complex64
-  PoolBuffer buf;
-  std::vector<cudaEvent_t> events;  // behind launches that read the buffer
+  PlanCopies<PlanApi> copies;   // of the matrices, one a device
 };
 
 // Tile bits by register size.  Small registers need tiles for every SM more than
@@ -403,42 +352,52 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
 
 void free_pass_plan(PassPlan *p) {
   if (!p) return;
-  p->buf.events = std::move(p->events);
-  give_buffer(p->buf);
+  std::string err;
+  PlanApi api{err};
+  p->copies.give_all(api, buffer_pool());
   delete p;
 }
 
 bool upload_pass_plan(PassPlan &p, std::string &err) {
   const size_t bytes = p.pool.size() * sizeof(double) + p.pool32.size() * sizeof(float);
-  if (p.buf.ptr || !bytes) return true;
+  int dev = 0;
+  if (!bytes) return true;
+  if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return false;
+  if (p.copies.on(dev)) return true;
   const void *src = p.pool.empty() ? (const void *)p.pool32.data() : (const void *)p.pool.data();
   RelaxedCapture relaxed;
-  static std::once_flag once;
-  static cudaError_t attr_rc = cudaSuccess;
-  std::call_once(once, [] {
-    attr_rc = cudaFuncSetAttribute(k_gate_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(sizeof(double2) << kPassMaxTile));
-    if (attr_rc == cudaSuccess)
-      attr_rc = cudaFuncSetAttribute(k_gate_pass32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(2 * kPass32MatBytes + (sizeof(float2) << kPass32MaxTile)));
-  });
-  if (!cuda_ok(attr_rc, "cudaFuncSetAttribute(gate pass kernel)", err)) return false;
-  PoolBuffer b;
-  if (!take_buffer(bytes, b, err)) return false;
+  // the shared-memory limit is a kernel's on one device
+  if (!cuda_ok(cudaFuncSetAttribute(k_gate_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(sizeof(double2) << kPassMaxTile)),
+               "cudaFuncSetAttribute(gate pass kernel)", err) ||
+      !cuda_ok(cudaFuncSetAttribute(k_gate_pass32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(2 * kPass32MatBytes + (sizeof(float2) << kPass32MaxTile))),
+               "cudaFuncSetAttribute(gate pass kernel)", err))
+    return false;
+  PlanApi api{err};
+  PlanBuffer<PlanApi> b;
+  if (!buffer_pool().take(api, dev, bytes, b)) return false;
   if (!upload_now(b.ptr, src, bytes, err)) {
-    give_buffer(b);
+    buffer_pool().give(api, std::move(b));
     return false;
   }
-  p.buf = std::move(b);
+  p.copies.add(std::move(b));
   return true;
 }
 
 bool launch_pass_plan(PassPlan &p, const std::vector<GateData> &gates, void *sv, uint32_t n,
                       cudaStream_t s, std::string &err) {
+  int dev = 0;
+  if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return false;
+  const PlanBuffer<PlanApi> *const mats = p.copies.on(dev);
   for (size_t i = 0; i < p.passes.size(); ++i) {
     if (p.arg_of[i] < 0) {
       if (!launch_gate(gates[p.passes[i].gates[0]], sv, n, s, err)) return false;
       continue;
+    }
+    if (!mats) {
+      err = "gate pass matrices are not on the current device";
+      return false;
     }
     const uint32_t tb = p.args.empty() ? p.args32[p.arg_of[i]].tb : p.args[p.arg_of[i]].tb;
     const uint64_t tiles = 1ull << (n - tb);
@@ -448,28 +407,23 @@ bool launch_pass_plan(PassPlan &p, const std::vector<GateData> &gates, void *sv,
     }
     if (p.args.empty())
       k_gate_pass32<<<(unsigned)tiles, kPassThreads, 2 * kPass32MatBytes + (sizeof(float2) << tb), s>>>(
-          static_cast<float2 *>(sv), reinterpret_cast<const float *>(p.buf.ptr), p.args32[p.arg_of[i]]);
+          static_cast<float2 *>(sv), reinterpret_cast<const float *>(mats->ptr), p.args32[p.arg_of[i]]);
     else
       k_gate_pass<<<(unsigned)tiles, kPassThreads, sizeof(double2) << tb, s>>>(
-          static_cast<double2 *>(sv), reinterpret_cast<const double *>(p.buf.ptr), p.args[p.arg_of[i]]);
+          static_cast<double2 *>(sv), reinterpret_cast<const double *>(mats->ptr), p.args[p.arg_of[i]]);
     if (!cuda_ok(cudaGetLastError(), "gate pass kernel launch", err)) return false;
   }
   return true;
 }
 
 bool mark_pass_plan(PassPlan &p, cudaStream_t s, std::string &err) {
-  if (!p.buf.ptr) return true;
+  int dev = 0;
+  if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return false;
+  PlanBuffer<PlanApi> *const mats = p.copies.on(dev);
+  if (!mats) return true;
   RelaxedCapture relaxed;
-  // an event that has completed is recorded again, so the list is as long as the
-  // most runs ever in flight at once
-  cudaEvent_t ev = nullptr;
-  for (size_t i = 0; i < p.events.size() && i < 8 && !ev; ++i)
-    if (cudaEventQuery(p.events[i]) == cudaSuccess) ev = p.events[i];
-  if (!ev) {
-    if (!cuda_ok(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate", err)) return false;
-    p.events.push_back(ev);
-  }
-  return cuda_ok(cudaEventRecord(ev, s), "cudaEventRecord (gate pass)", err);
+  PlanApi api{err};
+  return mats->mark(api, s);
 }
 
 }  // namespace cb2

@@ -116,9 +116,10 @@ uint32_t gate_choice_epoch();  // changes whenever such a choice is set
 
 // Merged passes (gate_pass.cu): a program's gates grouped into passes over the
 // statevector.  make_pass_plan touches no device; upload_pass_plan puts the
-// matrices on the device (synchronous, not under stream capture);
-// launch_pass_plan enqueues every pass; mark_pass_plan records, behind launches
-// on `s`, that the plan's device memory is in use until then.
+// matrices on the current device, once for each device the plan runs on
+// (synchronous, not under stream capture); launch_pass_plan enqueues every pass;
+// mark_pass_plan records, behind launches on `s`, that the plan's memory on the
+// current device is in use until then.
 struct Pass;
 struct PassPlan;
 std::vector<Pass> program_passes(const std::vector<GateData> &gates, uint32_t n);
