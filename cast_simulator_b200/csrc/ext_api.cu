@@ -404,9 +404,13 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
     const bool first = !plain && use_graph && s && p->graphs.find(key) == p->graphs.end() &&
                        p->ran.insert(key).second;
     if (!use_graph || !s || p->gates.empty() || first) {
-      if (!(plain ? p->launch_all(sv_dptr, s, err)
-                  : cb2::launch_pass_plan(*p->plans.back(), p->gates, sv, p->n, s, err) &&
-                        p->mark_plans(s, err))) {
+      // marked where a launch failed as well: the passes before it are queued
+      const bool launched = plain ? p->launch_all(sv_dptr, s, err)
+                                  : cb2::launch_pass_plan(*p->plans.back(), p->gates, sv, p->n, s, err);
+      std::string mark_err;
+      const bool marked = plain || p->mark_plans(s, mark_err);
+      if (launched && !marked) err = mark_err;
+      if (!launched || !marked) {
         write_err(err_buf, err_buf_len, err);
         return 1;
       }

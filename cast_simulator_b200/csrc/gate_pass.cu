@@ -183,6 +183,9 @@ struct PlanApi {
     return cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate (gate pass)", err);
   }
   void destroy(Event e) { cudaEventDestroy(e); }
+  bool id(Stream s, unsigned long long &id) {
+    return cuda_ok(cudaStreamGetId(s, &id), "cudaStreamGetId (gate pass)", err);
+  }
   bool allocate(size_t bytes, char *&p) {
     return cuda_ok(cudaMalloc((void **)&p, bytes), "cudaMalloc (gate pass matrices)", err);
   }
@@ -423,7 +426,9 @@ bool mark_pass_plan(PassPlan &p, cudaStream_t s, std::string &err) {
   if (!mats) return true;
   RelaxedCapture relaxed;
   PlanApi api{err};
-  return mats->mark(api, s);
+  if (mats->mark(api, s)) return true;
+  cudaStreamSynchronize(s);  // nothing keeps the buffer for what is queued: wait for it here
+  return false;
 }
 
 }  // namespace cb2

@@ -4,6 +4,7 @@
 //
 // Api: types Event and Stream, and
 //   bool done(Event), bool record(Event, Stream), bool create(Event &), void destroy(Event)
+//   bool id(Stream, unsigned long long &)     a stream's own, never used again
 //   bool allocate(size_t, char *&), void release(char *)      on the current device
 #pragma once
 
@@ -18,27 +19,42 @@ template <class Api> struct PlanBuffer {
   int device = 0;
   char *ptr = nullptr;
   size_t bytes = 0;
-  std::vector<typename Api::Event> events;  // behind launches that read it
+  // One event a stream, behind the last launch there that reads the buffer.  Streams
+  // are told apart by id: a handle may come back as another stream while the work of
+  // the one that had it is still in flight.
+  struct Reader {
+    unsigned long long stream;
+    typename Api::Event event;
+  };
+  std::vector<Reader> readers;
 
-  // Records that launches on `s` up to here read the buffer.
+  // Records that launches on `s` up to here read the buffer.  A new stream takes over
+  // the event of one whose work is done, so there are at most as many as streams ever
+  // had such work in flight at once, however many runs are queued on each.
   bool mark(Api &api, typename Api::Stream s) {
-    typename Api::Event ev{};
-    bool have = false;
-    for (size_t i = 0; i < events.size() && i < 8 && !have; ++i)
-      if (api.done(events[i])) ev = events[i], have = true;
-    if (!have) {
-      if (!api.create(ev)) return false;
-      events.push_back(ev);
+    unsigned long long id = 0;
+    if (!api.id(s, id)) return false;
+    Reader *at = nullptr;
+    for (Reader &r : readers)
+      if (r.stream == id) at = &r;
+    for (size_t i = 0; i < readers.size() && !at; ++i)
+      if (api.done(readers[i].event)) at = &readers[i];
+    if (!at) {
+      typename Api::Event e{};
+      if (!api.create(e)) return false;
+      readers.push_back(Reader{id, e});
+      at = &readers.back();
     }
-    return api.record(ev, s);
+    at->stream = id;
+    return api.record(at->event, s);
   }
 
   // True once every launch that reads the buffer has completed.
   bool settled(Api &api) {
-    while (!events.empty()) {
-      if (!api.done(events.back())) return false;
-      api.destroy(events.back());
-      events.pop_back();
+    while (!readers.empty()) {
+      if (!api.done(readers.back().event)) return false;
+      api.destroy(readers.back().event);
+      readers.pop_back();
     }
     return true;
   }
@@ -81,7 +97,7 @@ template <class Api> class PlanBufferPool {
       }
     }
     api.release(b.ptr);
-    for (auto &e : b.events) api.destroy(e);
+    for (auto &r : b.readers) api.destroy(r.event);
   }
 
  private:

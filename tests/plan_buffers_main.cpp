@@ -16,6 +16,7 @@ struct Fake {
   std::map<Event, bool> pending;      // recorded and not yet reached
   std::map<Event, Stream> on;         // stream of the last record
   std::map<char *, int> owner;        // allocation -> device
+  std::map<Stream, unsigned long long> ids;  // of handles that were used before
   char arena[64] = {};
   bool done(Event e) { return !pending[e]; }
   bool record(Event e, Stream s) {
@@ -29,6 +30,10 @@ struct Fake {
     return true;
   }
   void destroy(Event e) { live.erase(e); }
+  bool id(Stream s, unsigned long long &out) {
+    out = 100 * (unsigned long long)s + ids[s];
+    return true;
+  }
   bool allocate(size_t, char *&p) {
     p = &arena[next_ptr++];
     owner[p] = device;
@@ -93,7 +98,7 @@ int readers() {
   CHECK(pool.take(api, 0, 1000, b) && b.ptr != first);
   api.finish(2);
   CHECK(pool.take(api, 0, 1000, c) && c.ptr == first);
-  CHECK(c.events.empty() && api.live.empty());
+  CHECK(c.readers.empty() && api.live.empty());
   // over the pool's limit a buffer is released (which waits), with its events
   cb2::PlanBufferPool<Fake> none(0);
   CHECK(c.mark(api, 3));
@@ -102,9 +107,36 @@ int readers() {
   return 0;
 }
 
+// Runs queued by the hundred, between waits, on a few streams: as many events as
+// streams; and a stream handle that comes back while its old work runs gets its own.
+int events() {
+  Fake api;
+  cb2::PlanBufferPool<Fake> pool(1 << 20);
+  Buffer b, c;
+  CHECK(pool.take(api, 0, 1000, b));
+  for (int loop = 0; loop < 50; ++loop) {
+    for (int run = 0; run < 20; ++run)
+      for (int s = 1; s <= 3; ++s) CHECK(b.mark(api, s));
+    for (int s = 1; s <= 3; ++s) api.finish(s);
+  }
+  CHECK(b.readers.size() == 3 && api.made == 3);
+  CHECK(b.mark(api, 7) && api.made == 3);  // takes over the event of a finished one
+  ++api.ids[7];                            // destroyed with work in flight, handle reused
+  const Fake::Event old = b.readers[0].event;
+  CHECK(api.pending[old] && api.on[old] == 7);
+  CHECK(b.mark(api, 7) && b.readers[0].event == old);
+  int in_flight = 0;
+  for (auto &r : b.readers) in_flight += !api.done(r.event);
+  CHECK(in_flight == 2);
+  pool.give(api, std::move(b));
+  CHECK(pool.take(api, 0, 1000, c) && c.readers.empty());
+  return 0;
+}
+
 int main(int, char **argv) {
   const std::string what = argv[1];
   if (what == "devices") return devices();
   if (what == "readers") return readers();
+  if (what == "events") return events();
   return 2;
 }

@@ -17,7 +17,7 @@ def main(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("what", ["devices", "readers"])
+@pytest.mark.parametrize("what", ["devices", "readers", "events"])
 def test_plan_buffers(main, what):
     r = subprocess.run([main, what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout
