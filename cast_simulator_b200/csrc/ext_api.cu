@@ -57,11 +57,10 @@ struct Program {
   std::vector<GateData> gates;
   std::map<std::pair<uint64_t, void *>, cudaGraphExec_t> graphs;
   std::set<std::pair<uint64_t, void *>> ran;  // (statevector, stream) pairs run once
-  // How the gates are grouped into passes, newest last.  A changed kernel choice
-  // makes a new plan; graphs captured from an older one still read its matrices,
-  // so it stays until the graphs go.
-  std::vector<cb2::PassPlan *> plans;
-  uint32_t plan_epoch = 0;  // kernel choices the newest plan was made under
+  // How the gates are grouped into passes.  A changed kernel choice makes a new plan
+  // and drops the graphs captured from the old one with it.
+  cb2::PassPlan *plan = nullptr;
+  uint32_t plan_epoch = 0;  // kernel choices the plan was made under
   std::mutex mu;
 
   ~Program() {
@@ -73,25 +72,21 @@ struct Program {
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
     ran.clear();
-    for (cb2::PassPlan *p : plans) cb2::free_pass_plan(p);
-    plans.clear();
+    cb2::free_pass_plan(plan);
+    plan = nullptr;
   }
 
   bool ensure_plan(std::string &err) {
     const uint32_t epoch = cb2::gate_choice_epoch();
-    if (plans.empty() || plan_epoch != epoch) {
-      cb2::PassPlan *p = cb2::make_pass_plan(gates, n);
-      plans.push_back(p);
+    if (plan && plan_epoch != epoch) drop_graphs();
+    if (!plan) {
+      plan = cb2::make_pass_plan(gates, n);
       plan_epoch = epoch;
     }
-    return cb2::upload_pass_plan(*plans.back(), err);
+    return cb2::upload_pass_plan(*plan, err);
   }
 
-  bool mark_plans(cudaStream_t s, std::string &err) {
-    for (cb2::PassPlan *p : plans)
-      if (!cb2::mark_pass_plan(*p, s, err)) return false;
-    return true;
-  }
+  bool mark_plan(cudaStream_t s, std::string &err) { return !plan || cb2::mark_pass_plan(*plan, s, err); }
 
   // Gate after gate, each on its own kernel: for a stream that is being captured,
   // where nothing may be allocated and a caller's graph may outlive this program.
@@ -406,9 +401,9 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
     if (!use_graph || !s || p->gates.empty() || first) {
       // marked where a launch failed as well: the passes before it are queued
       const bool launched = plain ? p->launch_all(sv_dptr, s, err)
-                                  : cb2::launch_pass_plan(*p->plans.back(), p->gates, sv, p->n, s, err);
+                                  : cb2::launch_pass_plan(*p->plan, p->gates, sv, p->n, s, err);
       std::string mark_err;
-      const bool marked = plain || p->mark_plans(s, mark_err);
+      const bool marked = plain || p->mark_plan(s, mark_err);
       if (launched && !marked) err = mark_err;
       if (!launched || !marked) {
         write_err(err_buf, err_buf_len, err);
@@ -427,7 +422,7 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
         return 1;
       }
       const bool launched = plain ? p->launch_all(sv_dptr, s, err)
-                                  : cb2::launch_pass_plan(*p->plans.back(), p->gates, sv, p->n, s, err);
+                                  : cb2::launch_pass_plan(*p->plan, p->gates, sv, p->n, s, err);
       const cudaError_t end_rc = cudaStreamEndCapture(s, &graph);
       if (!launched || !cuda_ok(end_rc, "cudaStreamEndCapture", err) ||
           !cuda_ok(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate", err)) {
@@ -438,7 +433,7 @@ int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use
       cudaGraphDestroy(graph);
       it = p->graphs.emplace(key, exec).first;
     }
-    if (!cuda_ok(cudaGraphLaunch(it->second, s), "cudaGraphLaunch", err) || !p->mark_plans(s, err)) {
+    if (!cuda_ok(cudaGraphLaunch(it->second, s), "cudaGraphLaunch", err) || !p->mark_plan(s, err)) {
       write_err(err_buf, err_buf_len, err);
       return 1;
     }

@@ -88,3 +88,47 @@ def test_sparse_gates_in_passes(n, prec):
     st.sync()
     bound = 18 * 8 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
     assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
+
+
+def test_a_changed_choice_replaces_plan_and_graphs():
+    """A program that has a graph runs the grouping its plan() reports after a kernel
+    choice changes, and the old one again after it is taken back."""
+    from cast_simulator_b200.simulator import set_kernel_choice
+
+    n, prec = 12, CudaPrecision.F64
+    psi, gates = O.random_state(n, 4), _random_gates(n, 20, (3,), 5)
+    st, sv = Stream(), CudaStatevector(n, prec)
+
+    def program():
+        prog = GateProgram(prec, n, 1e-12, 1e-12)
+        for g in gates:
+            prog.add(g.matrix(), g.qubits())
+        return prog
+
+    def state(prog):
+        sv.upload(psi)
+        prog.run(sv, st)
+        st.sync()
+        return sv.download()
+
+    prog = program()
+    merged = [state(prog) for _ in range(3)]  # direct, captured, replayed
+    assert all(np.array_equal(m, merged[0]) for m in merged)
+    masks = {sum(1 << q for q in g.qubits() if q < 5) for g in gates} - {0}
+    for m in masks:
+        set_kernel_choice(prec, 3, m, "register")
+    try:
+        alone = state(program())
+        assert not np.array_equal(alone, merged[0])  # other roundings: the test can tell them apart
+        for _ in range(3):
+            assert np.array_equal(state(prog), alone)
+    finally:
+        for m in masks:
+            set_kernel_choice(prec, 3, m, None)
+    for _ in range(3):
+        assert np.array_equal(state(prog), merged[0])
+    want = psi.copy()
+    for g in gates:
+        O.apply_gate(want, g.matrix(), g.qubits())
+    for got in (merged[0], alone):
+        assert np.abs(got - want).max() <= 20 * 16 * 2.3e-16
