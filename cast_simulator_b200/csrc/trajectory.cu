@@ -1,6 +1,7 @@
 // Batched Monte-Carlo quantum-jump trajectories: programs, their upload and runs
 // (the kernels' device side is trajectory.cuh).
 #include "../../include/cast_b200.h"
+#include "seg_plan.hpp"
 #include "trajectory.cuh"
 
 #include <algorithm>
@@ -23,13 +24,6 @@ __global__ void __launch_bounds__(NT, 1)
 }
 
 constexpr uint32_t kTrajMagic = 0xCB2077A1u;
-
-// Threads per CTA when the program does not fix them: 1024 for states of 15 to
-// 17 qubits (slices larger than L1 but held in L2, so passes are bound by loads
-// in flight), 512 otherwise (issue-bound gate arithmetic).
-// A program with merged segments takes 512 for every size: their passes hold tiles
-// in shared memory, and their gate code needs the registers.
-unsigned auto_threads(uint32_t n, bool segments) { return !segments && n >= 15 && n <= 17 ? 1024u : 512u; }
 
 // Trajectories in flight when the program does not fix them: one per SM, unless
 // the slices of one per SM overflow L2 while those of at least half as many
@@ -125,6 +119,7 @@ struct TrajProgram {
   void *d_segs = nullptr;     // the segments' arrays, one buffer
   size_t segs_bytes = 0;
   TSegs segs{};
+  double width = 0;           // mean qubits of the GATE ops
   TRun *d_run = nullptr;
   double *d_z = nullptr;
   uint32_t *d_sample = nullptr;
@@ -132,7 +127,7 @@ struct TrajProgram {
   cudaGraphExec_t graph = nullptr;
   void *graph_stream = nullptr;
   unsigned graph_grid = 0;
-  unsigned threads = 0;  // threads per CTA: 512, 1024, or 0 for auto_threads(n)
+  unsigned threads = 0;  // threads per CTA: 512, 1024, or 0 for the size's own
   unsigned max_ctas = 0; // CTAs (trajectories in flight), or 0 for auto_ctas(n)
   unsigned graph_threads = 0;
   std::mutex mu;
@@ -174,8 +169,7 @@ struct TrajProgram {
     }
   }
 
-  // Groups every run of GATE ops into passes and uploads the segments that come out
-  // with fewer passes than gates.
+  // Plans the program's segments (seg_plan.cpp) and uploads them.
   bool build_segments(std::string &err) {
     std::vector<TSeg> sg;
     std::vector<TSegPass> ps;
@@ -184,16 +178,32 @@ struct TrajProgram {
     std::vector<float> mats;
     uint32_t mat_cap = 0;
     const uint32_t tb_most = std::min(n, kSegMaxTile);
+    std::vector<cb2::SegBlock> blocks;
+    std::vector<uint32_t> at;  // block -> its op
+    for (size_t i = 0; i < ops.size(); ++i) {
+      if (ops[i].type == T_GATE) {
+        cb2::SegBlock b;
+        for (uint32_t j = 0; j < ops[i].k; ++j) b.qubits |= 1ull << ops[i].q[j];
+        b.follows = i > 0 && (ops[i - 1].type == T_GATE || ops[i - 1].type == T_ERR);
+        blocks.push_back(b);
+        at.push_back((uint32_t)i);
+      } else if (ops[i].type == T_ERR && !blocks.empty()) {
+        blocks.back().quiet *= 1.0 - (double)ops[i].prob;
+      }
+    }
+    width = cb2::mean_width(blocks);
+    std::vector<cb2::Segment> plan;
+    if (n >= kSegMinQubits) plan = cb2::plan_segments(blocks, n, tb_most, kSegLow);
     std::vector<uint32_t> starts(ops.size(), 0);
-    for (size_t i = 0; i < ops.size() && n >= kSegMinQubits; ++i) {
-      if (ops[i].type != T_GATE) continue;
-      size_t end = i;
+    for (const cb2::Segment &seg : plan) {
       std::vector<cb2::GateData> gates;
       TSeg g{};
       g.err0 = (uint32_t)sites.size();
-      for (; end < ops.size() && (ops[end].type == T_GATE || ops[end].type == T_ERR); ++end) {
+      const uint32_t first_op = at[seg.first];
+      uint32_t end = first_op;
+      for (; end < ops.size() && (ops[end].type == T_ERR || gates.size() < seg.count); ++end) {
         if (ops[end].type == T_ERR) {
-          sites.push_back((uint32_t)end);
+          sites.push_back(end);
           continue;
         }
         cb2::GateData x;
@@ -213,23 +223,11 @@ struct TrajProgram {
         gates.push_back(std::move(x));
       }
       g.n_err = (uint32_t)sites.size() - g.err0;
-      g.end_op = (uint32_t)end;
-      std::vector<cb2::PassGate> pg(gates.size());
-      for (size_t j = 0; j < gates.size(); ++j) {
-        for (uint32_t b = 0; b < gates[j].k; ++b) pg[j].qubits |= 1ull << gates[j].qubits[b];
-        pg[j].mergeable = true;
-      }
-      const std::vector<cb2::Pass> passes =
-          cb2::plan_passes(pg, n, tb_most, kSegLow, cb2::kMaxPassGates, 11);
-      if (passes.size() >= gates.size()) {
-        sites.resize(g.err0);
-        i = end - 1;
-        continue;
-      }
+      g.end_op = end;
       g.pass0 = (uint32_t)ps.size();
-      g.n_passes = (uint32_t)passes.size();
-      for (const cb2::Pass &x : passes) {
-        uint64_t tile = x.tile ? x.tile : pg[x.gates[0]].qubits | ((1ull << std::min(n, kSegLow)) - 1);
+      g.n_passes = (uint32_t)seg.passes.size();
+      for (const cb2::Pass &x : seg.passes) {
+        uint64_t tile = x.tile ? x.tile : blocks[seg.first + x.gates[0]].qubits | ((1ull << std::min(n, kSegLow)) - 1);
         for (uint32_t b = 0; b < n && (uint32_t)__builtin_popcountll(tile) < tb_most; ++b) tile |= 1ull << b;
         std::vector<uint32_t> qubits;
         for (uint32_t q = 0; q < n; ++q)
@@ -249,9 +247,8 @@ struct TrajProgram {
         mat_cap = std::max(mat_cap, t.mat_bytes);
         ps.push_back(t);
       }
-      starts[i] = (uint32_t)sg.size() + 1;
+      starts[first_op] = (uint32_t)sg.size() + 1;
       sg.push_back(g);
-      i = end - 1;
     }
     buf_free(d_segs, segs_bytes);
     d_segs = nullptr;
@@ -538,7 +535,9 @@ int cast_b200_traj_run_range(void *prog, uint32_t first, uint32_t n_traj, uint64
     }
     const unsigned ctas = p->max_ctas ? p->max_ctas : auto_ctas(p->n);
     const unsigned grid = (unsigned)std::min<uint64_t>(n_traj, ctas);
-    const unsigned threads = p->threads ? p->threads : auto_threads(p->n, p->segs.segs != nullptr);
+    // a program with segments: 512, for their tiles in shared memory and the registers
+    const unsigned threads = p->threads ? p->threads
+                             : p->segs.segs ? (unsigned)kTMinThreads : cb2::plain_threads(p->n, p->width);
     if (p->ws_ctas < grid) {
       buf_free(p->d_ws, p->ws_bytes);
       p->d_ws = nullptr;

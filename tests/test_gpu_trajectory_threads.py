@@ -39,3 +39,20 @@ def test_programs_of_different_sizes_run_in_threads(cblib, graph):
     for t in threads:
         t.join()
     assert not wrong, wrong[:4]
+
+
+@pytest.mark.parametrize("n,k,p", [(8, 2, 3e-2), (12, 3, 1e-2), (13, 4, 3e-3), (14, 2, 1e-2), (16, 3, 1e-2),
+                                   (17, 2, 3e-3)])
+def test_fired_pieces_match_the_plain_kernel(cblib, n, k, p):
+    """The same draws (depolarizing: they do not depend on the state) in passes where a
+    piece stays quiet, block by block where it fires, and block by block throughout."""
+    from cast_simulator_b200.trajectory import TrajectoryProgram
+    from cast_simulator_b200.types import QuantumCircuit
+
+    prog = TrajectoryProgram(QuantumCircuit.brickwork(n, 8, n, depolarizing=p), k)
+    blocks = sum(op[0] == "gate" for op in prog.ops())
+    z, _ = prog.run(24, 3)
+    prog.set_launch(1024, 0)  # the kernel without segments
+    plain, _ = prog.run(24, 3)
+    # a block is at most 16 FP32 products and sums an amplitude; fired sites add as many
+    assert np.abs(z - plain).max() <= 4 * blocks * 16 * 1.2e-7
