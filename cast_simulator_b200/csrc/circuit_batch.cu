@@ -70,7 +70,7 @@ struct BCircuit {
 struct alignas(16) BOp {
   uint32_t mat;  // byte offset of the matrix in the pool (16-byte aligned)
   uint32_t mat_bytes;
-  uint32_t k;    // of the gate, or of its laid-out form when resident
+  uint32_t k;
   uint32_t q[kBatchMaxGate];
   union {  // resident circuits: the walk of the tile
     cb2::PassGateArgs a64;
@@ -277,13 +277,20 @@ __device__ void run_resident(BShared &S, unsigned char *smem, const BOp *__restr
     const BOp &o = slots[oi & 1];
     if constexpr (F64) {
       const double *m = reinterpret_cast<const double *>(mat);
-      if (o.k == 4) cb2::pass_gate4_full<NT / 32>(s, m, o.a64, N >> 7, warp, lane);
-      else cb2::pass_gate3<NT / 32>(s, m, o.a64, N >> 6, warp, lane);
+      switch (o.k) {
+      case 4: cb2::pass_gate4_full<NT / 32>(s, m, o.a64, N >> 7, warp, lane); break;
+      case 3: cb2::pass_gate3<NT / 32>(s, m, o.a64, N >> 6, warp, lane); break;
+      case 2: cb2::pass_small<NT / 32, 2, 2>(s, m, o.a64, N >> 6, warp, lane); break;
+      default: cb2::pass_small<NT / 32, 1, 2>(s, m, o.a64, N >> 6, warp, lane);
+      }
     } else {
       const float *m = reinterpret_cast<const float *>(mat);
-      if (o.k == 4) cb2::pass_gate32<NT, 4, 2, 2, false>(s, m, o.a32, c.n);
-      else if (o.k == 3) cb2::pass_gate32<NT, 3, 1, 2, false>(s, m, o.a32, c.n);
-      else cb2::pass_gate32<NT, 2, 1, 4, false>(s, m, o.a32, c.n);
+      switch (o.k) {
+      case 4: cb2::pass_gate32<NT, 4, 2, 2, false>(s, m, o.a32, c.n); break;
+      case 3: cb2::pass_gate32<NT, 3, 1, 2, false>(s, m, o.a32, c.n); break;
+      case 2: cb2::pass_gate32<NT, 2, 1, 4, false>(s, m, o.a32, c.n); break;
+      default: cb2::pass_gate32<NT, 1, 1, 4, false>(s, m, o.a32, c.n);
+      }
     }
   }
   __syncthreads();
@@ -411,8 +418,7 @@ bool add_circuit(Batch &b, uint64_t sv, uint32_t n, uint8_t prec, uint32_t n_gat
     const void *from = prec ? (const void *)g.m64.data() : (const void *)g.m32.data();
     if (c.resident) {
       for (uint32_t j = 0; j < k; ++j) g.qubits[j] = op.q[j];
-      const cb2::PlacedGate placed = cb2::place_gate(g, tile_qubits, prec ? 3 : 2);
-      op.k = placed.k;
+      const cb2::PlacedGate placed = cb2::place_gate(g, tile_qubits);
       frag64.clear();
       frag32.clear();
       if (prec) cb2::pack_gate(placed, n, false, frag64, op.a64);

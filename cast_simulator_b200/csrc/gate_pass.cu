@@ -45,6 +45,10 @@ struct PassArgs {
   PassGateArgs g[kMaxPassGates];
 };
 
+// NARROW: the pass has gates of 1 or 2 qubits.  Their code and the tests that lead to
+// it cost the other gates of small states 25 to 40 ns each (17 qubits, fused at 3:
+// 96 -> 105 us), so passes without them run without it.
+template <bool NARROW>
 __global__ void __launch_bounds__(kPassThreads, 3)
     k_gate_pass(double2 *__restrict__ psi, const double *__restrict__ pool,
                 const __grid_constant__ PassArgs a) {
@@ -80,7 +84,9 @@ __global__ void __launch_bounds__(kPassThreads, 3)
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   for (uint32_t gi = 0; gi < a.n_gates; ++gi) {
     const PassGateArgs &g = a.g[gi];
-    if (g.k == 4) pass_gate4<kPassWarps>(s, pool + g.mat, g, tile >> 7, warp, lane);
+    if (NARROW && g.k == 2) pass_small<kPassWarps, 2, 2>(s, pool + g.mat, g, tile >> 6, warp, lane);
+    else if (NARROW && g.k == 1) pass_small<kPassWarps, 1, 4>(s, pool + g.mat, g, tile >> 6, warp, lane);
+    else if (g.k == 4) pass_gate4<kPassWarps>(s, pool + g.mat, g, tile >> 7, warp, lane);
     else if (g.k > 4)
       pass_sparse<kPassWarps>(s, reinterpret_cast<const double2 *>(pool + g.mat), g.k, g.sp, a.tb, warp, lane);
     else pass_gate3<kPassWarps>(s, pool + g.mat, g, tile >> 6, warp, lane);
@@ -114,6 +120,8 @@ struct PassArgs32 {
   PassGateArgs32 g[kMaxPassGates];
 };
 
+// NARROW: the pass has 1-qubit gates.
+template <bool NARROW>
 __global__ void __launch_bounds__(kPassThreads, 3)
     k_gate_pass32(float2 *__restrict__ psi, const float *__restrict__ pool,
                   const __grid_constant__ PassArgs32 a) {
@@ -156,7 +164,10 @@ __global__ void __launch_bounds__(kPassThreads, 3)
     if (gi + 1 < a.n_gates) fetch_matrix(gi + 1);
     const PassGateArgs32 &g = a.g[gi];
     const float *m = mat + (gi & 1) * (kPass32MatBytes / 4);
-    if (g.k == 4) pass_gate32<kPassThreads, 4, 2, 2, true>(s, m, g, a.tb);
+    if (NARROW && g.k == 1) {
+      if (a.tb > 9) pass_gate32<kPassThreads, 1, 1, 4, false>(s, m, g, a.tb);
+      else pass_gate32<kPassThreads, 1, 1, 2, false>(s, m, g, a.tb);  // 2 groups a thread at most
+    } else if (g.k == 4) pass_gate32<kPassThreads, 4, 2, 2, true>(s, m, g, a.tb);
     else if (g.k > 4)
       pass_sparse<kPassWarps>(s, reinterpret_cast<const float2 *>(pool + g.mat), g.k, g.sp, a.tb,
                               __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), (int)threadIdx.x & 31);
@@ -328,7 +339,7 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
           a.g[i].k = (uint16_t)g.k;
           pack_sparse(g, qubits, pass_swz, p->pool, a.g[i].mat, a.g[i].sp);
         } else {
-          pack_gate(place_gate(g, qubits, 3), tb, g.k == 4, p->pool, a.g[i]);
+          pack_gate(place_gate(g, qubits), tb, g.k == 4, p->pool, a.g[i]);
         }
       }
     } else {
@@ -344,7 +355,7 @@ PassPlan *make_pass_plan(const std::vector<GateData> &gates, uint32_t n) {
           a.g[i].k = (uint16_t)g.k;
           pack_sparse(g, qubits, pass_swz32, p->pool32, a.g[i].mat, a.g[i].sp);
         } else {
-          pack_gate32(place_gate(g, qubits, 2), tb, g.k == 4, p->pool32, a.g[i]);
+          pack_gate32(place_gate(g, qubits), tb, g.k == 4, p->pool32, a.g[i]);
         }
       }
     }
@@ -370,12 +381,13 @@ bool upload_pass_plan(PassPlan &p, std::string &err) {
   const void *src = p.pool.empty() ? (const void *)p.pool32.data() : (const void *)p.pool.data();
   RelaxedCapture relaxed;
   // the shared-memory limit is a kernel's on one device
-  if (!cuda_ok(cudaFuncSetAttribute(k_gate_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(sizeof(double2) << kPassMaxTile)),
-               "cudaFuncSetAttribute(gate pass kernel)", err) ||
-      !cuda_ok(cudaFuncSetAttribute(k_gate_pass32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(2 * kPass32MatBytes + (sizeof(float2) << kPass32MaxTile))),
-               "cudaFuncSetAttribute(gate pass kernel)", err))
+  auto opt_in = [&](auto kernel, size_t most) {
+    return cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most),
+                   "cudaFuncSetAttribute(gate pass kernel)", err);
+  };
+  const size_t most64 = sizeof(double2) << kPassMaxTile, most32 = 2 * kPass32MatBytes + (sizeof(float2) << kPass32MaxTile);
+  if (p.pool.empty() ? !opt_in(k_gate_pass32<false>, most32) || !opt_in(k_gate_pass32<true>, most32)
+                     : !opt_in(k_gate_pass<false>, most64) || !opt_in(k_gate_pass<true>, most64))
     return false;
   PlanApi api{err};
   PlanBuffer<PlanApi> b;
@@ -408,12 +420,20 @@ bool launch_pass_plan(PassPlan &p, const std::vector<GateData> &gates, void *sv,
       err = "statevector too large for the gate pass kernel grid";
       return false;
     }
-    if (p.args.empty())
-      k_gate_pass32<<<(unsigned)tiles, kPassThreads, 2 * kPass32MatBytes + (sizeof(float2) << tb), s>>>(
-          static_cast<float2 *>(sv), reinterpret_cast<const float *>(mats->ptr), p.args32[p.arg_of[i]]);
-    else
-      k_gate_pass<<<(unsigned)tiles, kPassThreads, sizeof(double2) << tb, s>>>(
-          static_cast<double2 *>(sv), reinterpret_cast<const double *>(mats->ptr), p.args[p.arg_of[i]]);
+    auto narrow = [](const auto &a, uint32_t below) {
+      return std::any_of(a.g, a.g + a.n_gates, [&](const auto &g) { return g.k < below; });
+    };
+    if (p.args.empty()) {
+      const PassArgs32 &a = p.args32[p.arg_of[i]];
+      const auto kernel = narrow(a, 2) ? k_gate_pass32<true> : k_gate_pass32<false>;
+      kernel<<<(unsigned)tiles, kPassThreads, 2 * kPass32MatBytes + (sizeof(float2) << tb), s>>>(
+          static_cast<float2 *>(sv), reinterpret_cast<const float *>(mats->ptr), a);
+    } else {
+      const PassArgs &a = p.args[p.arg_of[i]];
+      const auto kernel = narrow(a, 3) ? k_gate_pass<true> : k_gate_pass<false>;
+      kernel<<<(unsigned)tiles, kPassThreads, sizeof(double2) << tb, s>>>(
+          static_cast<double2 *>(sv), reinterpret_cast<const double *>(mats->ptr), a);
+    }
     if (!cuda_ok(cudaGetLastError(), "gate pass kernel launch", err)) return false;
   }
   return true;

@@ -37,9 +37,11 @@ struct SparseGateArgs {
 
 // One gate of a pass.  Index contributions are swizzled tile offsets; XOR of the
 // contributions of an index's set bits is its place in shared memory.
+// k = 1, 2: ld_k holds the member bits, ld_lane (4 of it for k = 2) and blk the group
+// bits; the st_ fields are unused.
 struct PassGateArgs {
   uint32_t mat;          // first double of its fragments in the pool
-  uint16_t k;            // 3 or 4; 5..7 for a sparse gate
+  uint16_t k;            // 1..4; 5..7 for a sparse gate
   uint16_t ld_lane[5];   // load: lane bits 0, 1 -> member bits 0, 1; 2..4 -> group bits 0..2
   uint16_t ld_k[2];      // load: member bits 2, 3 (the k steps)
   uint16_t st_lane[5];   // store: lane bits 0, 1 -> group bits 1, 2; 2..4 -> row bits 0..2
@@ -215,13 +217,66 @@ __device__ __forceinline__ void pass_gate3(double2 *s, const double *mat, const 
   for (; round * W + warp < n_blk; ++round) pass_gate3_blocks<W, 1>(s, c, d, g, ld, st, wb, round);
 }
 
+// 1- and 2-qubit gates: a lane a gather group, or half the rows of one (2 qubits: two
+// lanes of a warp read the same amplitudes, and hold half a matrix each), the fma
+// sequence of the one-gate kernels.  (Padded with the identity to the 3-qubit form they
+// took twice the arithmetic, and its zeros spread an infinity to amplitudes the gate
+// leaves alone.)  U rounds at once keep loads in flight.
+template <int W, int K, int U>
+__device__ __forceinline__ void pass_small_rounds(double2 *s, const double2 (&m)[K == 1 ? 4 : 8],
+                                                  const PassGateArgs &g, uint32_t lb, uint32_t top,
+                                                  uint32_t round) {
+  constexpr int D = 1 << K, R = 2;  // rows a lane
+  uint32_t off[D], bx[U];
+  double2 x[U][D];
+#pragma unroll
+  for (int a = 0; a < D; ++a) off[a] = (a & 1 ? g.ld_k[0] : 0) ^ (a & 2 ? g.ld_k[1] : 0);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    bx[u] = lb ^ round_bits<W>(g, round + u);
+#pragma unroll
+    for (int a = 0; a < D; ++a) x[u][a] = s[bx[u] ^ off[a]];
+  }
+  if (K == 2) __syncwarp();  // the partner has read these groups
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      double re = 0.0, im = 0.0;
+#pragma unroll
+      for (int c = 0; c < D; ++c) {
+        const double2 e = m[r * D + c];
+        re = fma(e.x, x[u][c].x, re);
+        re = fma(-e.y, x[u][c].y, re);
+        im = fma(e.x, x[u][c].y, im);
+        im = fma(e.y, x[u][c].x, im);
+      }
+      s[bx[u] ^ top ^ off[r]] = make_double2(re, im);
+    }
+}
+
+// n_blk: blocks of 32 groups (k = 1) or 16 (k = 2).
+template <int W, int K, int U>
+__device__ __forceinline__ void pass_small(double2 *s, const double *mat, const PassGateArgs &g, uint32_t n_blk, int warp, int lane) {
+  constexpr int E = K == 1 ? 4 : 8;
+  const bool half = K == 2 && lane >= 16;
+  double2 m[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) m[e] = reinterpret_cast<const double2 *>(mat)[e + (half ? E : 0)];
+  const uint32_t lb = lane_bits(g.ld_lane, lane) ^ warp_bits<W>(g, warp), top = half ? g.ld_k[1] : 0;
+  uint32_t round = 0;
+  for (; (round + U - 1) * W + warp < n_blk; round += U) pass_small_rounds<W, K, U>(s, m, g, lb, top, round);
+  if (U > 1)
+    for (; round * W + warp < n_blk; ++round) pass_small_rounds<W, K, 1>(s, m, g, lb, top, round);
+}
+
 constexpr uint32_t kPass32MatBytes = 3 * 256 * sizeof(float);
 
 struct PassGateArgs32 {
   uint32_t mat;           // first float of its columns in the pool
-  uint16_t k;             // 2..4; 5..7 for a sparse gate
+  uint16_t k;             // 1..4; 5..7 for a sparse gate
   uint16_t member[4];     // gate bits
-  uint16_t group[kTileMax32 - 2];  // group bits (a 2-qubit gate has the most)
+  uint16_t group[kTileMax32 - 1];  // group bits (a 1-qubit gate has the most)
   SparseGateArgs sp;      // k >= 5
 };
 
@@ -247,7 +302,7 @@ template <int K, int H, int U, bool M3>
 __device__ __forceinline__ void pass_groups32(float2 *s, const float *mat, const PassGateArgs32 &g,
                                               const uint32_t (&gb)[U], uint32_t half, bool live) {
   constexpr int D = 1 << K, P = D / 2 / H, S = M3 ? 3 : 2;  // row pairs, sums a row pair
-  const float4 *m = reinterpret_cast<const float4 *>(mat) + half * (3 * P / 2);
+  const float2 *m = reinterpret_cast<const float2 *>(mat) + half * (3 * P);
   float2 acc[U][S][P];
 #pragma unroll
   for (int u = 0; u < U; ++u)
@@ -267,17 +322,24 @@ __device__ __forceinline__ void pass_groups32(float2 *s, const float *mat, const
       const float sum = x.x + x.y;
       xs[u] = make_float2(sum, sum);
     }
+    constexpr int Q = P < 2 ? 1 : 2;  // row pairs at once: two are three 16-byte loads
 #pragma unroll
-    for (int h = 0; h < P / 2; ++h) {  // two row pairs: three 16-byte loads
-      const float4 *mc = m + 3 * (c * (D / 4) + h);
-      const float4 m0 = mc[0], m1 = mc[1], m2 = mc[2];
-      const float2 e[2][3] = {{make_float2(m0.x, m0.y), make_float2(m0.z, m0.w), make_float2(m1.x, m1.y)},
-                              {make_float2(m1.z, m1.w), make_float2(m2.x, m2.y), make_float2(m2.z, m2.w)}};
+    for (int h = 0; h < P / Q; ++h) {
+      const float2 *mc = m + 3 * (c * (D / 2) + Q * h);
+      float2 e[Q][3];
+      if constexpr (Q == 2) {
+        const float4 *m4 = reinterpret_cast<const float4 *>(mc);
+        const float4 m0 = m4[0], m1 = m4[1], m2 = m4[2];
+        e[0][0] = make_float2(m0.x, m0.y), e[0][1] = make_float2(m0.z, m0.w), e[0][2] = make_float2(m1.x, m1.y);
+        e[1][0] = make_float2(m1.z, m1.w), e[1][1] = make_float2(m2.x, m2.y), e[1][2] = make_float2(m2.z, m2.w);
+      } else {  // a 1-qubit gate
+        e[0][0] = mc[0], e[0][1] = mc[1], e[0][2] = mc[2];
+      }
 #pragma unroll
-      for (int q = 0; q < 2; ++q)
+      for (int q = 0; q < Q; ++q)
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-          const int p = 2 * h + q;
+          const int p = Q * h + q;
           if constexpr (M3) {
             acc[u][0][p] = __ffma2_rn(e[q][0], xs[u], acc[u][0][p]);
             acc[u][1][p] = __ffma2_rn(e[q][1], xr[u], acc[u][1][p]);
@@ -322,11 +384,11 @@ __device__ __forceinline__ void pass_gate32(float2 *s, const float *mat, const P
   auto offset = [&](uint32_t group, int from, int to) {  // group bits from .. to - 1
     uint32_t o = 0;
 #pragma unroll
-    for (int b = 0; b < (int)kTileMax32 - 2; ++b)
+    for (int b = 0; b < (int)kTileMax32 - 1; ++b)
       if (b >= from && b < to && ((group >> b) & 1)) o ^= g.group[b];
     return o;
   };
-  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0, LAST = (int)kTileMax32 - 2;
+  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0, LAST = (int)kTileMax32 - 1;
   static_assert(U == 1 << LU, "a power of two of groups");
   const uint32_t groups = 1u << (tb - K), t = offset(gt, 0, TB);
   if (groups >= U * GT) {
@@ -536,49 +598,19 @@ inline void pack_sparse(const GateData &g, const std::vector<uint32_t> &tile_qub
   }
 }
 
-// The gate on k' = max(least, k) tile positions: positions (ascending, member bit b
-// at pos[b]) and the matrix, padded with the identity on spare positions.
+// The gate's places in the tile (ascending, member bit b at pos[b]) and its matrix.
 struct PlacedGate {
   uint32_t k = 0;
   uint32_t pos[4] = {0};
-  const double *m = nullptr;   // interleaved, 2^k x 2^k: the gate's own, or `padded`
-  std::vector<double> padded;
+  const double *m = nullptr;   // interleaved, 2^k x 2^k
 };
 
-inline PlacedGate place_gate(const GateData &g, const std::vector<uint32_t> &tile_qubits, uint32_t least) {
+inline PlacedGate place_gate(const GateData &g, const std::vector<uint32_t> &tile_qubits) {
   PlacedGate p;
-  auto position = [&](uint32_t q) {
-    return (uint32_t)(std::lower_bound(tile_qubits.begin(), tile_qubits.end(), q) - tile_qubits.begin());
-  };
-  uint32_t pos[4] = {0}, used = 0;
-  for (uint32_t b = 0; b < g.k; ++b) used |= 1u << (pos[b] = position(g.qubits[b]));
-  for (uint32_t c = (uint32_t)tile_qubits.size(); (uint32_t)__builtin_popcount(used) < least && c-- > 0;) used |= 1u << c;
-  for (uint32_t c = 0; c < tile_qubits.size(); ++c)
-    if ((used >> c) & 1) p.pos[p.k++] = c;
-  if (p.k == g.k) {
-    p.m = g.m64.data();
-    return p;
-  }
-  const uint32_t D = 1u << p.k;
-  uint32_t gate_bit[4] = {0}, gate_mask = 0;  // bit of the padded index holding gate bit b
-  for (uint32_t b = 0; b < g.k; ++b) {
-    gate_bit[b] = (uint32_t)__builtin_popcount(used & ((1u << pos[b]) - 1));
-    gate_mask |= 1u << gate_bit[b];
-  }
-  p.padded.assign(2 * D * D, 0.0);
-  for (uint32_t r = 0; r < D; ++r)
-    for (uint32_t c = 0; c < D; ++c) {
-      if ((r ^ c) & ~gate_mask) continue;
-      uint32_t gr = 0, gc = 0;
-      for (uint32_t b = 0; b < g.k; ++b) {
-        gr |= ((r >> gate_bit[b]) & 1) << b;
-        gc |= ((c >> gate_bit[b]) & 1) << b;
-      }
-      const size_t src = 2 * (((size_t)gr << g.k) + gc), dst = 2 * ((size_t)r * D + c);
-      p.padded[dst] = g.m64[src];
-      p.padded[dst + 1] = g.m64[src + 1];
-    }
-  p.m = p.padded.data();
+  p.k = g.k;
+  p.m = g.m64.data();
+  for (uint32_t b = 0; b < g.k; ++b)
+    p.pos[b] = (uint32_t)(std::lower_bound(tile_qubits.begin(), tile_qubits.end(), g.qubits[b]) - tile_qubits.begin());
   return p;
 }
 
@@ -637,10 +669,38 @@ inline LaneOrder lane_order(const PlacedGate &p, uint32_t tb) {
   return o;
 }
 
+// A 1- or 2-qubit gate: its matrix as it is, and group bits such that the 8 lanes of a
+// wavefront fall into different bank groups (three lane bits that differ mod 3).
+inline void pack_small(const PlacedGate &p, uint32_t tb, std::vector<double> &pool, PassGateArgs &out) {
+  std::memset(&out, 0, sizeof(out));
+  out.mat = (uint32_t)pool.size();
+  out.k = (uint16_t)p.k;
+  pool.insert(pool.end(), p.m, p.m + ((size_t)2 << (2 * p.k)));
+  uint32_t order[kTileMax64], n_order = 0, used = 0;
+  for (uint32_t b = 0; b < p.k; ++b) used |= 1u << p.pos[b];
+  auto take = [&](uint32_t c) {
+    order[n_order++] = c;
+    used |= 1u << c;
+  };
+  for (uint32_t cls = 0; cls < 3; ++cls)
+    for (uint32_t c = cls; c < tb; c += 3)
+      if (!((used >> c) & 1)) {
+        take(c);
+        break;
+      }
+  for (uint32_t c = 0; c < tb; ++c)
+    if (!((used >> c) & 1)) take(c);
+  auto at = [](uint32_t position) { return (uint16_t)pass_swz(1u << position); };
+  const uint32_t lanes = p.k == 1 ? 5 : 4;
+  for (uint32_t b = 0; b < n_order; ++b) (b < lanes ? out.ld_lane[b] : out.blk[b - lanes]) = at(order[b]);
+  for (uint32_t b = 0; b < p.k; ++b) out.ld_k[b] = at(p.pos[b]);
+}
+
 // Appends a gate's A fragments to the pool (lane l holds row l / 4 and column
 // l % 4 of an 8 x 4 block) and fills its launch arguments.
 // `three`: the three-product form (4-qubit gates).
 inline void pack_gate(const PlacedGate &p, uint32_t tb, bool three, std::vector<double> &pool, PassGateArgs &out) {
+  if (p.k < 3) return pack_small(p, tb, pool, out);
   const LaneOrder o = lane_order(p, tb);
   const uint32_t D = 1u << p.k;
   uint32_t row_of[16], col_of[16];

@@ -240,7 +240,7 @@ struct TrajProgram {
         for (uint32_t j = 0; j < t.tb; ++j) t.stride[j] = 1u << qubits[j];
         for (const uint32_t j : x.gates) {
           cb2::PassGateArgs32 a;
-          cb2::pack_gate32(cb2::place_gate(gates[j], qubits, 2), t.tb, false, mats, a);
+          cb2::pack_gate32(cb2::place_gate(gates[j], qubits), t.tb, false, mats, a);
           gs.push_back(a);
         }
         t.mat_bytes = (uint32_t)((mats.size() - t.mat) * sizeof(float));

@@ -552,9 +552,12 @@ struct Traj {
           } else if (g.k == 3) {
             cb2::pass_gate32<NT, 3, 1, 2, false>(s, m, g, tb);
             m += 3 * 64;
-          } else {
+          } else if (g.k == 2) {
             cb2::pass_gate32<NT, 2, 1, 4, false>(s, m, g, tb);
             m += 3 * 16;
+          } else {
+            cb2::pass_gate32<NT, 1, 1, 4, false>(s, m, g, tb);
+            m += 3 * 4;
           }
           __syncthreads();
         }

@@ -132,3 +132,44 @@ def test_a_changed_choice_replaces_plan_and_graphs():
         O.apply_gate(want, g.matrix(), g.qubits())
     for got in (merged[0], alone):
         assert np.abs(got - want).max() <= 20 * 16 * 2.3e-16
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("widths", [(1,), (2,), (1, 2, 3, 4)])
+@pytest.mark.parametrize("prec", [CudaPrecision.F64, CudaPrecision.F32])
+@pytest.mark.parametrize("path", ["program", "batch"])
+def test_an_infinity_stays_in_its_groups(path, prec, widths, bad):
+    """An amplitude that is not finite reaches the amplitudes that gates on its qubits
+    mix it with, and no others."""
+    from cast_simulator_b200.simulator import CircuitBatch
+
+    n, acted, at = 10, [1, 4, 5, 8], 0b1011010110
+    rng = np.random.default_rng(len(widths))
+    gates = [T.QuantumGate.random_unitary(sorted(int(q) for q in rng.choice(acted, size=widths[i % len(widths)],
+                                                                             replace=False)), rng)
+             for i in range(12)]
+    psi = O.random_state(n, 6)
+    want = psi.copy()
+    want[at] = 0
+    for g in gates:
+        O.apply_gate(want, g.matrix(), g.qubits())
+    psi[at] = bad
+    sv, st = CudaStatevector(n, prec), Stream()
+    sv.upload(psi)
+    if path == "program":
+        prog = GateProgram(prec, n, 0.0, 0.0)
+        for g in gates:
+            prog.add(g.matrix(), g.qubits())
+        assert len(set(prog.plan()[0].tolist())) < len(gates)
+        prog.run(sv, st)
+        st.sync()
+    else:
+        batch = CircuitBatch()
+        batch.add(sv, gates, init_zero=False)
+        batch.run(st)
+    mask = sum(1 << q for q in acted)
+    apart = (np.arange(1 << n) ^ at) & ~mask != 0  # never in a group with the bad one
+    got = sv.download()[apart]
+    assert np.isfinite(got).all()
+    bound = 12 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
+    assert np.abs(got - want[apart]).max() <= bound
