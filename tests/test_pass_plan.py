@@ -76,3 +76,83 @@ def test_forced_kernel_choices_are_not_merged():
     finally:
         set_kernel_choice(CudaPrecision.F64, 3, 0b111, None)
     assert len(set(prog.plan()[0].tolist())) == merged
+
+
+def _greedy(masks, n, tb, low, most):
+    """The grouping as a plain restatement: every seed grown to the end, every count a
+    walk over the whole window."""
+    out, pending = [], list(range(len(masks)))
+    low_mask = (1 << min(low, n)) - 1
+
+    def scan(q):
+        taken, ready, blocked = [], [], 0
+        for i in pending[:128]:
+            if not masks[i] & blocked:
+                if not masks[i] & ~q and len(taken) < most:
+                    taken.append(i)
+                    continue
+                if masks[i] & ~q:
+                    ready.append(masks[i])
+            blocked |= masks[i]
+        return taken, ready
+
+    while pending:
+        taken, ready = scan(low_mask)
+        best, tile = [], 0
+        for seed in ready + ([low_mask] if taken else []):
+            q = low_mask | seed
+            if q.bit_count() > tb:
+                continue
+            taken, around = scan(q)
+            while True:
+                grow, gain, added = 0, 0, 1
+                for x in around:
+                    if (q | x).bit_count() <= tb:
+                        more = len(scan(q | x)[0]) - len(taken)
+                        add = (q | x).bit_count() - q.bit_count()
+                        if more > 0 and (not grow or more * added > gain * add):
+                            grow, gain, added = q | x, more, add
+                if not grow:
+                    break
+                q = grow
+                taken, around = scan(q)
+            if len(taken) > len(best):
+                best, tile = taken, q
+        if len(best) < 2:
+            best = pending[:1]
+        out.append(best)
+        pending = [i for i in pending if i not in set(best)]
+    return out
+
+
+@pytest.mark.parametrize("n,widths,spread", [(9, (1,), True), (12, (1, 2), False), (14, (1, 2, 3, 4), True),
+                                             (17, (2, 1), True), (20, (1, 1, 2), False)])
+def test_plan_is_the_greedy_grouping(n, widths, spread):
+    gates = _gates(n, 160, widths, n, spread)
+    which, place = _program(n, CudaPrecision.F64, gates).plan()
+    masks = [sum(1 << q for q in g.qubits()) for g in gates]
+    tile = min(n, 11, max(9, n - 8))  # of complex128 states below 22 qubits
+    want = _greedy(masks, n, tile, 3, 16)
+    got = [[] for _ in range(int(which.max()) + 1)]
+    for i in np.lexsort((place, which)):
+        got[which[i]].append(int(i))
+    assert got == want
+
+
+def test_long_programs_are_planned_quickly():
+    """Planning is paid in a program's first run: it grows with the gates, not with
+    their number times what waits behind them (50000 took 0.9 s)."""
+    import time
+
+    n, x = 20, T.QuantumGate.random_unitary([0], np.random.default_rng(1)).matrix()
+    prog = GateProgram(CudaPrecision.F64, n, 0.0, 0.0)
+    for i in range(50000):
+        prog.add(x, [i % n])
+    best = min(_timed(prog.plan, time.perf_counter) for _ in range(3))
+    assert best < 0.3
+
+
+def _timed(f, clock):
+    t = clock()
+    f()
+    return clock() - t
