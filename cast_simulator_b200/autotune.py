@@ -341,7 +341,8 @@ def tune_kernels(n: int = 26, precisions=("f64", "f32"), ks=range(1, 5), reps: i
     each candidate's milliseconds.  A tile kernel wins only when it beats the
     register kernel by more than ``margin`` (the launch-to-launch spread).  With
     ``apply`` the winners are routed process-wide, else every class goes back to
-    the built-in rule."""
+    the built-in rule; they hold where a gate runs alone, and programs go on
+    merging gates into passes."""
     from .cuda import CudaPrecision, CudaStatevector
     from .simulator import Stream, gate_engine, set_kernel_choice
 
@@ -364,7 +365,7 @@ def tune_kernels(n: int = 26, precisions=("f64", "f32"), ks=range(1, 5), reps: i
                                   key=lambda x: x[1])
             if best > ms["register"] * (1.0 - margin):
                 eng, tb = "register", 0
-            set_kernel_choice(prec, k, mask, eng if apply else None, tb if apply else 0)
+            set_kernel_choice(prec, k, mask, eng if apply else None, tb if apply else 0, forced=False)
             out.append({"precision": pname, "k": k, "low_mask": mask, "targets": list(q),
                         "engine": eng, "tile_bits": tb, "builtin": builtin, "ms": ms})
         del sv
@@ -389,7 +390,8 @@ def cxx_table(choices) -> str:
 
 def apply_kernel_choices(choices) -> int:
     """Route the classes of ``choices`` (``tune_kernels`` records, or a
-    ``HardwareProfile`` holding them) process-wide; returns how many."""
+    ``HardwareProfile`` holding them) process-wide, for gates that run alone;
+    returns how many."""
     from .cuda import CudaPrecision
     from .simulator import set_kernel_choice
 
@@ -397,7 +399,7 @@ def apply_kernel_choices(choices) -> int:
         choices = choices.kernel_choices
     for c in choices:
         prec = CudaPrecision.F64 if c["precision"] == "f64" else CudaPrecision.F32
-        set_kernel_choice(prec, c["k"], c["low_mask"], c["engine"], c["tile_bits"])
+        set_kernel_choice(prec, c["k"], c["low_mask"], c["engine"], c["tile_bits"], forced=False)
     return len(choices)
 
 

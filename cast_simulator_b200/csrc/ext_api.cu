@@ -102,6 +102,17 @@ Program *as_program(void *p) {
   return pr && pr->magic == kProgramMagic ? pr : nullptr;
 }
 
+int store_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int engine, uint32_t tile_bits,
+                 bool forced, char *err_buf, size_t err_buf_len) {
+  std::string err;
+  if (!cb2::set_kernel_choice(precision, k, low_mask, engine, tile_bits, forced, err)) {
+    write_err(err_buf, err_buf_len, err);
+    return 1;
+  }
+  clear_err(err_buf, err_buf_len);
+  return 0;
+}
+
 __global__ void k_set_one(void *p, int f64) {
   if (f64) *static_cast<double *>(p) = 1.0;
   else *static_cast<float *>(p) = 1.0f;
@@ -181,13 +192,12 @@ int cast_b200_set_gate_path(int path) { return cb2::set_gate_path(path); }
 
 int cast_b200_set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int engine,
                                 uint32_t tile_bits, char *err_buf, size_t err_buf_len) {
-  std::string err;
-  if (!cb2::set_kernel_choice(precision, k, low_mask, engine, tile_bits, err)) {
-    write_err(err_buf, err_buf_len, err);
-    return 1;
-  }
-  clear_err(err_buf, err_buf_len);
-  return 0;
+  return store_choice(precision, k, low_mask, engine, tile_bits, true, err_buf, err_buf_len);
+}
+
+int cast_b200_prefer_kernel(uint8_t precision, uint32_t k, uint32_t low_mask, int engine,
+                            uint32_t tile_bits, char *err_buf, size_t err_buf_len) {
+  return store_choice(precision, k, low_mask, engine, tile_bits, false, err_buf, err_buf_len);
 }
 
 int cast_b200_gate_engine(uint8_t precision, uint32_t sv_n_qubits, const cast_complex64_t *matrix,

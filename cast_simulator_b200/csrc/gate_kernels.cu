@@ -936,13 +936,15 @@ std::atomic<int> g_gate_path{[] {
 
 int gate_path_override() { return g_gate_path.load(std::memory_order_relaxed); }
 
-// Per-class kernel choices written by the autotuner (cast_b200_set_kernel_choice).
+// Per-class kernel choices (cast_b200_set_kernel_choice, and cast_b200_prefer_kernel
+// for the autotuner's, which leave merging alone).
 // A class is (precision, k = 1..4, the mask of targets below qubit 5).  engine:
 // -1 the built-in rule below, 0 register kernel, 1 tile kernel; tile_bits: 0 the
 // built-in size, 11 or 12 (2048 / 4096 amplitudes a tile).
 struct KernelChoice {
   std::atomic<int> engine{-1};
   std::atomic<int> tile_bits{0};
+  std::atomic<bool> forced{false};  // the class is kept out of merged passes
 };
 KernelChoice g_choice[2][5][32];
 std::atomic<uint32_t> g_choice_epoch{0};
@@ -1014,7 +1016,7 @@ int set_gate_path(int path) {
 }
 
 bool set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int engine,
-                       uint32_t tile_bits_, std::string &err) {
+                       uint32_t tile_bits_, bool forced, std::string &err) {
   if (precision > 1 || k < 1 || k > 4 || low_mask == 0 || low_mask > 31 ||
       (uint32_t)__builtin_popcount(low_mask) > k || engine < -1 || engine > 1 ||
       (tile_bits_ != 0 && tile_bits_ != 11 && tile_bits_ != 12)) {
@@ -1025,6 +1027,7 @@ bool set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int eng
   KernelChoice &c = g_choice[precision][k][low_mask];
   c.engine.store(engine);
   c.tile_bits.store((int)tile_bits_);
+  c.forced.store(forced && (engine >= 0 || tile_bits_));
   ++g_choice_epoch;
   return true;
 }
@@ -1035,7 +1038,7 @@ bool gate_choice_forced(const GateData &g) {
   uint32_t low_bits = 0;
   for (uint32_t b = 0; b < g.k; ++b)
     if (g.qubits[b] < 5) low_bits |= 1u << g.qubits[b];
-  return low_bits && g_choice[g.precision ? 1 : 0][g.k][low_bits].engine.load(std::memory_order_relaxed) >= 0;
+  return low_bits && g_choice[g.precision ? 1 : 0][g.k][low_bits].forced.load(std::memory_order_relaxed);
 }
 
 int sm_count() {

@@ -103,14 +103,14 @@ int set_tensor_loader(int mode);
 // Device helpers shared between translation units.
 int sm_count();
 int set_gate_path(int path);  // 0 auto, 1 register, 2 tile; returns previous
-// Autotuned choice for dense gates of k <= 4 with targets below qubit 5 (see
-// cast_b200_set_kernel_choice).
+// Choice for dense gates of k <= 4 with targets below qubit 5 (see
+// cast_b200_set_kernel_choice; not forced: cast_b200_prefer_kernel).
 bool set_kernel_choice(uint8_t precision, uint32_t k, uint32_t low_mask, int engine,
-                       uint32_t tile_bits, std::string &err);
+                       uint32_t tile_bits, bool forced, std::string &err);
 bool upload_gate_matrix(GateData &g, std::string &err);  // fills g.d_mat
 
-// True while a kernel choice set from outside (a forced path or an autotuned
-// class) decides how this gate runs; such gates are not merged into passes.
+// True while a path or a choice forced from outside decides how this gate runs; such
+// gates are not merged into passes.
 bool gate_choice_forced(const GateData &g);
 uint32_t gate_choice_epoch();  // changes whenever such a choice is set
 

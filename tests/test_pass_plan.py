@@ -5,7 +5,7 @@ import pytest
 
 from cast_simulator_b200 import types as T
 from cast_simulator_b200.cuda import CudaPrecision
-from cast_simulator_b200.simulator import GateProgram, set_kernel_choice
+from cast_simulator_b200.simulator import GateProgram, gate_engine, set_kernel_choice
 from oracle import oracle as O
 
 TILE = 13  # qubits of the largest tile
@@ -156,3 +156,36 @@ def _timed(f, clock):
     t = clock()
     f()
     return clock() - t
+
+
+def test_tuned_choices_leave_merging_alone():
+    from cast_simulator_b200 import autotune as A
+
+    n = 24
+    for prec, name in ((CudaPrecision.F64, "f64"), (CudaPrecision.F32, "f32")):
+        prog = _program(n, prec, T.QuantumCircuit.brickwork(n, 6, 1).gates())
+        plan = prog.plan()
+        recs = [{"precision": name, "k": k, "low_mask": m, "engine": e, "tile_bits": tb}
+                for (k, m), (e, tb) in zip(A.kernel_classes(), 99 * A.KERNEL_CANDIDATES)]
+        try:
+            assert A.apply_kernel_choices(recs) == len(recs)
+            assert np.array_equal(prog.plan(), plan)
+            # they do decide the kernel of a gate that runs alone
+            r = next(r for r in recs if r["k"] == 2 and r["engine"] == "tile")
+            q = A.class_targets(n, 2, r["low_mask"])
+            assert gate_engine(A.haar(2, np.random.default_rng(0)), q, n, prec) == "tile"
+        finally:
+            for r in recs:
+                set_kernel_choice(prec, r["k"], r["low_mask"], None)
+
+
+def test_a_chosen_tile_size_is_not_merged():
+    gates = _gates(12, 30, (3,), 1, False)
+    prog = _program(12, CudaPrecision.F64, gates)
+    low = [i for i, g in enumerate(gates) if tuple(g.qubits()) == (0, 1, 2)]
+    set_kernel_choice(CudaPrecision.F64, 3, 0b111, None, 12)  # the built-in kernel, another tile
+    try:
+        which = prog.plan()[0].tolist()
+        assert all(which.count(which[i]) == 1 for i in low)
+    finally:
+        set_kernel_choice(CudaPrecision.F64, 3, 0b111, None)
