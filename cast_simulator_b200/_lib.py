@@ -125,6 +125,8 @@ CAST_B200 = [
     ("cast_b200_set_tensor_loader", C.c_int, [C.c_int]),
     ("cast_b200_program_num_gates", C.c_uint32, [C.c_void_p]),
     ("cast_b200_program_plan", C.c_int, [C.c_void_p, c_u32p, c_u32p, C.c_char_p, C.c_size_t]),
+    ("cast_b200_fused_plan", C.c_int, [C.c_void_p, C.c_uint8, C.c_uint32, C.c_double, C.c_double, C.c_int, c_u32p,
+                                       C.c_char_p, C.c_size_t]),
     ("cast_b200_program_run", C.c_int,
      [C.c_void_p, C.c_uint64, C.c_void_p, C.c_int, C.c_char_p, C.c_size_t]),
     ("cast_b200_program_destroy", None, [C.c_void_p]),

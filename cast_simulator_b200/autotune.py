@@ -17,9 +17,10 @@ AI = peak / bw_slope to the hardware-adaptive cost model
     ``tensor_min_k = 5``, so ``HardwareProfile.crossover_for(k)`` gives the
     tensor-pipe crossover for wide gates;
   * ``choose_fusion`` fuses the circuit at every width k with the native
-    planner and predicts its time from the measured per-pass times (scaled by
-    2^(n - n_profile), the passes being memory-bound), then returns the width
-    and engine with the least predicted time;
+    planner, groups the gates into the passes a program would make of them and
+    predicts its time from measured times of gates that run alone and of gates
+    in a merged pass (scaled by 2^(n - n_profile)), then returns the width and
+    engine with the least predicted time;
   * ``tune_trajectories`` times the batched-trajectory kernel of a noisy
     circuit at each fusion width and launch shape (threads per CTA, CTAs in
     flight) and returns the fastest;
@@ -186,16 +187,27 @@ def measure_profile(n: int = 26, precision: str = "f32", ks=range(1, 8), reps: i
 
 @dataclass
 class PassTable:
-    """Measured seconds per pass, keyed by (k, mode), at ``n_qubits``."""
+    """Measured seconds per one-gate pass, keyed by (k, mode), at ``n_qubits``;
+    ``merged``: of a gate in a merged pass, keyed the same, and of the pass
+    itself (its copies and start) at ("pass", precision)."""
 
     n_qubits: int
     seconds: dict = field(default_factory=dict)
+    merged: dict = field(default_factory=dict)
 
     def predict(self, k: int, mode: str, n: int) -> float:
         key = (k, mode)
         if key not in self.seconds:
             raise KeyError(f"no measured pass time for k={k} mode={mode}")
         return self.seconds[key] * 2.0 ** (n - self.n_qubits)
+
+    def predict_pass(self, gates, precision: str, n: int) -> float:
+        """Seconds of one pass of ``gates``, (k, mode) each.  Gates that share a
+        pass are priced alone where the table has no merged times for them."""
+        if len(gates) > 1 and ("pass", precision) in self.merged and all(g in self.merged for g in gates):
+            t = self.merged["pass", precision] + sum(self.merged[g] for g in gates)
+            return t * 2.0 ** (n - self.n_qubits)
+        return sum(self.predict(k, mode, n) for k, mode in gates)
 
 
 def measure_pass_table(n: int, precision: str, ks=range(1, 8), tensor: bool = True,
@@ -210,7 +222,53 @@ def measure_pass_table(n: int, precision: str, ks=range(1, 8), tensor: bool = Tr
         for k in SPARSE_KS:
             if k in ks:
                 tab.seconds[(k, "s" + precision)] = time_gate(n, k, "s" + precision, reps=reps)
+    measure_merged(tab, precision, ks, sparse, reps)
     return tab
+
+
+def measure_merged(tab: PassTable, precision: str, ks, sparse: bool = True, reps: int = 3) -> None:
+    """Fills ``tab.merged``: programs of 4 and of 12 gates on the same qubits, one
+    pass each, give a gate's time by their difference; what the 4-gate program
+    takes besides its gates is the pass.  Gates that this size does not merge are left
+    out."""
+    per, start = {}, []
+    for k, mode in ([(k, precision) for k in ks if k <= 4]
+                    + [(k, "s" + precision) for k in SPARSE_KS if sparse and k in ks]):
+        t = [_time_merged(tab.n_qubits, k, mode, m, reps) for m in (4, 12)]
+        if None not in t:
+            per[k, mode] = max(0.0, (t[1] - t[0]) / 8)
+            start.append(t[0] - 4 * per[k, mode])
+    if per:
+        tab.merged.update(per)
+        tab.merged["pass", precision] = max(0.0, float(np.median(start)))
+
+
+def _time_merged(n: int, k: int, mode: str, count: int, reps: int, seed: int = 1):
+    """Seconds of a program of ``count`` k-qubit gates that shares one pass (best of
+    ``reps`` after one warm-up), or None where it does not."""
+    from .cuda import CudaPrecision, CudaStatevector
+    from .simulator import Event, GateProgram, Stream
+
+    if k > n:
+        return None
+    prec = CudaPrecision.F64 if mode in ("f64", "sf64") else CudaPrecision.F32
+    prog, rng = GateProgram(prec, n, 1e-12, 1e-12), np.random.default_rng(seed)
+    for _ in range(count):
+        prog.add(monomial(k, rng) if mode.startswith("s") else haar(k, rng), tuple(range(n - k, n)))
+    if len(set(prog.plan()[0].tolist())) > 1:
+        return None
+    sv, st = CudaStatevector(n, prec), Stream()
+    sv.zero()
+    e0, e1 = Event(), Event()
+    best = math.inf
+    for i in range(reps + 1):
+        e0.record(st)
+        prog.run(sv, st, use_graph=False)
+        e1.record(st)
+        e1.sync()
+        if i:
+            best = min(best, e1.elapsed_s(e0))
+    return best
 
 
 def engine_for(k: int, precision: str, split: bool, sparse: bool = False) -> str:
@@ -236,7 +294,8 @@ def choose_fusion(n: int, gates, precision: str, table: PassTable, ks=range(2, 7
     """Fuse ``gates`` at each width in ``ks`` (size-only cost, the reference's
     default) and predict the circuit time from ``table``; returns the width and
     engine (CUDA cores, or tensor cores for 5- and 6-qubit gates) with the least
-    predicted time.  Each fused gate is priced at the pass time of the kernel
+    predicted time.  The gates are grouped into the passes a program makes of them
+    (``FusedCircuit.plan``), and each is priced at the time of the kernel
     family the library routes it to (``simulator.gate_engine``): sparse gates at
     the table's "sf64" / "sf32" entries, split-precision tensor gates at "tc"."""
     from .cuda import CudaPrecision
@@ -247,15 +306,17 @@ def choose_fusion(n: int, gates, precision: str, table: PassTable, ks=range(2, 7
     cands = []
     splits = (False, True) if (allow_tensor and precision == "f32") else (False,)
     for k in ks:
-        fused = optimize_native(n, gates, FusionConfig.size_only(k)).gates()
+        circuit = optimize_native(n, gates, FusionConfig.size_only(k))
+        fused = circuit.gates()
         for split in splits:
-            # the library's own routing decides each gate's kernel family
-            t = sum(table.predict(g.n_qubits(),
-                                  mode_of.get(gate_engine(g.matrix(), g.qubits(), n, prec, split),
-                                              precision), n)
-                    for g in fused)
+            # the library's own routing decides each gate's kernel family and pass
+            passes: dict = {}
+            for g, p in zip(fused, circuit.plan(n, prec, split)):
+                mode = mode_of.get(gate_engine(g.matrix(), g.qubits(), n, prec, split), precision)
+                passes.setdefault(p, []).append((g.n_qubits(), mode))
+            t = sum(table.predict_pass(gs, precision, n) for gs in passes.values())
             cands.append({"fusion_k": k, "split_precision": split, "fused_gates": len(fused),
-                          "predicted_s": t})
+                          "passes": len(passes), "predicted_s": t})
     best = min(cands, key=lambda c: c["predicted_s"])
     return Choice(best["fusion_k"], best["split_precision"], best["predicted_s"], cands)
 

@@ -373,6 +373,43 @@ int cast_b200_program_plan(void *program, uint32_t *out_pass, uint32_t *out_plac
   }
 }
 
+int cast_b200_fused_plan(const void *fused, uint8_t precision, uint32_t n_qubits, double ztol, double otol,
+                         int split, uint32_t *out_pass, char *err_buf, size_t err_buf_len) {
+  try {
+    static char on_device;  // stands for a device copy: planning only asks whether there is one
+    std::vector<GateData> gates(cast_b200_fused_num_gates(fused));
+    std::string err;
+    std::vector<cast_complex64_t> m;
+    for (uint32_t i = 0; i < gates.size(); ++i) {
+      GateData &g = gates[i];
+      uint32_t k = 0, q[cb2::kMaxGateQubits] = {0};
+      bool ok = !cast_b200_fused_gate(fused, i, &k, q, nullptr) && k <= cb2::kMaxGateQubits;
+      if (ok) {
+        m.resize(size_t(1) << (2 * k));
+        cast_b200_fused_gate(fused, i, &k, q, m.data());
+        ok = make_gate(precision, m.data(), q, k, ztol, otol, g, err) && cb2::check_gate(g, n_qubits, err);
+      } else {
+        err = "fused gate is wider than the kernels take";
+      }
+      if (!ok) {
+        write_err(err_buf, err_buf_len, err);
+        return -1;
+      }
+      if (cb2::sparse_gate(g)) g.d_sparse = &on_device;
+      else if (split && cb2::tensor_path_supported(g)) g.d_tc = &on_device;
+    }
+    const std::vector<cb2::Pass> passes = cb2::program_passes(gates, n_qubits);
+    for (uint32_t i = 0; i < passes.size(); ++i)
+      for (const uint32_t j : passes[i].gates)
+        if (out_pass) out_pass[j] = i;
+    clear_err(err_buf, err_buf_len);
+    return (int)passes.size();
+  } catch (const std::exception &ex) {
+    write_err(err_buf, err_buf_len, ex.what());
+    return -1;
+  }
+}
+
 int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use_graph,
                           char *err_buf, size_t err_buf_len) {
   Program *p = as_program(program);

@@ -532,6 +532,21 @@ class FusedCircuit:
 
         return int(L.lib().cast_b200_fused_num_gates(self.handle))
 
+    def plan(self, n_qubits: int, precision: int, split_precision: bool = False, ztol: float = 1e-12,
+             otol: float = 1e-12) -> list[int]:
+        """The pass of every gate in a gate program made of this circuit
+        (cast_b200_fused_plan; touches no device)."""
+        import numpy as np
+
+        from . import _lib as L
+
+        out = np.zeros(max(1, len(self)), dtype=np.uint32)
+        eb = L.errbuf()
+        if L.lib().cast_b200_fused_plan(self.handle, int(precision), n_qubits, ztol, otol, int(split_precision),
+                                        out.ctypes.data_as(L.c_u32p), eb, L.ERR_LEN) < 0:
+            raise RuntimeError(f"fused_plan failed: {eb.value.decode()}")
+        return out[:len(self)].tolist()
+
     def gates(self) -> list[QuantumGate]:
         import ctypes as C
 

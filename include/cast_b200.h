@@ -136,6 +136,11 @@ int cast_b200_program_plan(void *program, uint32_t *out_pass, uint32_t *out_plac
                            size_t err_buf_len);
 int cast_b200_program_run(void *program, uint64_t sv_dptr, void *stream, int use_graph,
                           char *err_buf, size_t err_buf_len);
+/* The pass of every gate of a fused circuit in a program of n_qubits made of it
+ * (split: in split-precision mode); as cast_b200_program_plan, without the program
+ * and without a device. */
+int cast_b200_fused_plan(const void *fused, uint8_t precision, uint32_t n_qubits, double ztol, double otol,
+                         int split, uint32_t *out_pass, char *err_buf, size_t err_buf_len);
 void cast_b200_program_destroy(void *program);
 
 /* -- FP64 reductions ---------------------------------------------------------------

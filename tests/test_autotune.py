@@ -105,3 +105,38 @@ def test_choose_fusion_prefers_the_fastest_predicted_engine(cblib):
     with pytest.raises(KeyError):
         dear_tc.predict(7, "tc", n)
     assert all(math.isfinite(c["predicted_s"]) for c in ch.candidates)
+
+
+def test_fused_plan_is_the_programs(cblib):
+    from cast_simulator_b200.cuda import CudaPrecision
+    from cast_simulator_b200.fusion import FusionConfig, optimize_native
+    from cast_simulator_b200.simulator import GateProgram
+
+    n = 24
+    fused = optimize_native(n, _brickwork(n, 10), FusionConfig.size_only(4))
+    for prec in (CudaPrecision.F64, CudaPrecision.F32):
+        prog = GateProgram(prec, n, 1e-12, 1e-12)
+        for g in fused.gates():
+            prog.add(g.matrix(), g.qubits())
+        assert fused.plan(n, prec) == prog.plan()[0].tolist()
+    wide = optimize_native(n, _brickwork(n, 10), FusionConfig.size_only(6))
+    ids = wide.plan(n, CudaPrecision.F32, split_precision=True)
+    sizes = [g.n_qubits() for g in wide.gates()]
+    assert all(ids.count(p) == 1 for p, k in zip(ids, sizes) if k >= 5)  # tensor gates run alone
+
+
+def test_choose_fusion_sees_merged_passes(cblib):
+    """Wide gates win on times of gates that run alone; merged passes, which only gates
+    of up to 4 qubits make, turn that round."""
+    n = 24
+    gates = _brickwork(n, 10)
+    alone = {(k, "f64"): t for k, t in zip(range(1, 8), (1.0, 1.0, 1.0, 1.1, 1.5, 2.0, 6.0))}
+    assert A.choose_fusion(n, gates, "f64", A.PassTable(n, dict(alone))).fusion_k >= 5
+    merged = {(k, "f64"): t for k, t in zip(range(1, 5), (0.1, 0.15, 0.3, 0.55))}
+    tab = A.PassTable(n, dict(alone), {**merged, ("pass", "f64"): 0.9})
+    ch = A.choose_fusion(n, gates, "f64", tab)
+    assert ch.fusion_k <= 4
+    best = next(c for c in ch.candidates if c["fusion_k"] == ch.fusion_k)
+    assert best["passes"] < best["fused_gates"]
+    assert tab.predict_pass([(4, "f64")], "f64", n) == pytest.approx(1.1)  # a gate alone in its pass
+    assert tab.predict_pass([(4, "f64"), (2, "f64")], "f64", n + 1) == pytest.approx(2 * (0.9 + 0.55 + 0.15))
