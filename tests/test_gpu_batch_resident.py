@@ -45,3 +45,27 @@ def test_batch_matches_oracle(sizes, prec):
         idx = np.arange(1 << n)
         want_z = [1 - 2 * p[(idx >> q) & 1 == 1].sum() / p.sum() for q in range(n)]
         assert np.abs(got_z - want_z).max() <= 4 * bound
+
+
+@pytest.mark.parametrize("prec", [CudaPrecision.F64, CudaPrecision.F32])
+def test_a_refused_circuit_leaves_the_batch_as_it_was(prec):
+    st, batch = Stream(), CircuitBatch()
+    svs = [CudaStatevector(n, prec) for n in (9, 8, 12)]
+    gates = [_circuit(n, 9, n) for n in (9, 8, 12)]
+    batch.add(svs[0], gates[0])
+    wide = T.QuantumGate.random_unitary([0, 1, 2, 3, 4], np.random.default_rng(0))
+    outside = T.QuantumGate.random_unitary([7, 8], np.random.default_rng(0))
+    for bad in (wide, outside):
+        with pytest.raises(RuntimeError):
+            batch.add(svs[1], gates[1] + [bad])
+        assert len(batch) == 1
+    batch.run(st)
+    batch.add(svs[2], gates[2])  # after a run: the tables go up again
+    z = batch.run(st)
+    assert [len(x) for x in z] == [9, 12]
+    bound = 9 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
+    for sv, gs in ((svs[0], gates[0]), (svs[2], gates[2])):
+        psi = O.zero_state(sv.n_qubits())
+        for g in gs:
+            O.apply_gate(psi, g.matrix(), g.qubits())
+        assert np.abs(sv.download() - psi).max() <= bound
