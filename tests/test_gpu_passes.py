@@ -45,12 +45,13 @@ def test_program_matches_oracle(n, widths, graph, prec):
         prog.add(g.matrix(), g.qubits())
         O.apply_gate(want, g.matrix(), g.qubits())
     sv, st = CudaStatevector(n, prec), Stream()
-    sv.upload(psi)
-    prog.run(sv, st, use_graph=graph)
-    st.sync()
     # 24 unitary gates: each adds at most a few units of 2^k roundings
     bound = 24 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
-    assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
+    for _ in range(3 if graph else 1):  # a direct run, the captured one, a replay
+        sv.upload(psi)
+        prog.run(sv, st, use_graph=graph)
+        st.sync()
+        assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
 
 
 def _sparse_gate(n, k, per_row, rng):
@@ -83,11 +84,12 @@ def test_sparse_gates_in_passes(n, prec):
         prog.add(g.matrix(), g.qubits())
         O.apply_gate(want, g.matrix(), g.qubits())
     sv, st = CudaStatevector(n, prec), Stream()
-    sv.upload(psi)
-    prog.run(sv, st)
-    st.sync()
     bound = 18 * 8 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
-    assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
+    for _ in range(3):  # a direct run, the captured one, a replay
+        sv.upload(psi)
+        prog.run(sv, st)
+        st.sync()
+        assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
 
 
 def test_a_changed_choice_replaces_plan_and_graphs():
@@ -173,3 +175,64 @@ def test_an_infinity_stays_in_its_groups(path, prec, widths, bad):
     assert np.isfinite(got).all()
     bound = 12 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
     assert np.abs(got - want[apart]).max() <= bound
+
+
+@pytest.mark.parametrize("prec", [CudaPrecision.F64, CudaPrecision.F32])
+def test_under_a_callers_capture(prec):
+    """On a stream that the caller captures, a program enqueues gate after gate and
+    allocates nothing; the caller's graph replays it."""
+    import torch
+
+    n = 12
+    psi, gates = O.random_state(n, 8), _random_gates(n, 20, (1, 2, 3, 4), 9)
+    prog, want = GateProgram(prec, n, 0.0, 0.0), psi.copy()
+    for g in gates:
+        prog.add(g.matrix(), g.qubits())
+        O.apply_gate(want, g.matrix(), g.qubits())
+    sv, graph, side = CudaStatevector(n, prec), torch.cuda.CUDAGraph(), torch.cuda.Stream()
+
+    class Captured:
+        handle = side.cuda_stream
+
+    bound = 20 * 16 * (2.3e-16 if prec == CudaPrecision.F64 else 1.2e-7)
+    with torch.cuda.graph(graph, stream=side):
+        prog.run(sv, Captured, use_graph=False)
+    for _ in range(2):
+        sv.upload(psi)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
+    sv.upload(psi)  # and in passes again outside the capture
+    prog.run(sv, Captured, use_graph=False)
+    torch.cuda.synchronize()
+    assert np.abs(sv.download() - want).max() <= bound * np.abs(want).max()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_dropped_programs_matrices_stay_until_its_launches_end(graph):
+    """Programs dropped with their launches queued, each followed by another that could
+    take its buffer."""
+    n, prec = 22, CudaPrecision.F64
+    st, other = Stream(), Stream()
+    a, b = CudaStatevector(n, prec), CudaStatevector(n, prec)
+    psi = O.random_state(n, 2)
+    a.upload(psi)
+    b.upload(psi)
+    want_a, want_b = psi.copy(), psi.copy()
+    for j in range(4):
+        for sv, stream, want, runs in ((a, st, want_a, 3), (b, other, want_b, 1)):
+            gates = _random_gates(n, 6, (3, 4), 10 * j + runs)
+            prog = GateProgram(prec, n, 1e-12, 1e-12)
+            for g in gates:
+                prog.add(g.matrix(), g.qubits())
+            for _ in range(runs):
+                prog.run(sv, stream, use_graph=graph)
+                for g in gates:
+                    O.apply_gate(want, g.matrix(), g.qubits())
+            del prog  # its launches are still queued
+    st.sync()
+    other.sync()
+    bound = 4 * 3 * 6 * 16 * 2.3e-16
+    assert np.abs(a.download() - want_a).max() <= bound
+    assert np.abs(b.download() - want_b).max() <= bound

@@ -59,6 +59,10 @@ def test_qft_cx_program_graph_and_eager(mods, oracle):
     st.sync()
     ref2 = oracle.simulate(n, _oracle_gates(circ), ref)
     assert np.max(np.abs(sv.download() - ref2)) < 1e-10
+    sv.upload(init)
+    prog.run(sv, st)  # a replay of the graph the second run captured
+    st.sync()
+    assert np.max(np.abs(sv.download() - ref)) < 1e-10
 
 
 @pytest.mark.parametrize("path", [1, 2])
