@@ -13,6 +13,9 @@ reference's size-only fusion at width k (default 4), complex128 statevector
            src/profile.rs:427-436).
   e2e    : same metric through the public Simulator API per step: gate
            matrices uploaded from host, run, <Z_q> for every qubit read back.
+           A program's gates share passes over the state, so the metric (one
+           read and one write a fused gate) is no HBM traffic there and can
+           exceed the card's rate; passes_per_step and hbm_gbs say what moves.
   roofline / cpu_baseline / clocks: see the JSON keys.
 
 Keys beside the headline (rank 0, one GPU): c2_complex64 (the same 30-qubit
@@ -206,7 +209,7 @@ def cpu_parity(n: int, depth: int, k: int, precision: str, threads: int) -> dict
     _, gates = build_fused(n, depth, k)
     ref = cpu_reference_state(n, gates, threads)
     prec = cu.CudaPrecision.F64 if precision == "f64" else cu.CudaPrecision.F32
-    _, gsv = _run_fused(n, gates, prec, reps=1)
+    _, gsv, _ = _run_fused(n, gates, prec, reps=1)
     psi = gsv.download()
     rep = fidelity_vs(ref, psi)
     return {"workload": f"brickwork-{n}q-d{depth} fused k={k} ({len(gates)} passes), from |0>",
@@ -293,12 +296,24 @@ def _random_state(n: int, seed: int) -> np.ndarray:
     return v / np.linalg.norm(v)
 
 
+def _program_rates(n: int, gates: int, passes: int, amp: int, t: float) -> dict:
+    """Rates of a gate program: gate_gbs counts one read and one write of the state
+    per fused gate (the headline metric's accounting), hbm_gbs one per pass the
+    program makes of them, which is what moves."""
+    state = 2 * (1 << n) * amp / 1e9
+    return {"state_passes": passes, "gate_gbs": gates * state / t, "hbm_gbs": passes * state / t}
+
+
+def _passes(prog) -> int:
+    return len(set(prog.plan()[0].tolist()))
+
+
 def _run_fused(n: int, gates, precision, split: bool = False, initial=None, reps: int = 3,
                warm: bool = True, use_graph: bool = True):
     """Device time (median of reps, CUDA events) of a fused gate list as one
-    gate program, and the final statevector object.  With `warm`, one untimed
-    run first (graph capture, first launches); every timed run starts from the
-    same initial state."""
+    gate program, the final statevector object and the passes the program makes.
+    With `warm`, untimed runs first (first launches, graph capture); every timed
+    run starts from the same initial state."""
     from cast_simulator_b200 import cuda as cu
     from cast_simulator_b200.simulator import Event, GateProgram, Stream
 
@@ -310,7 +325,8 @@ def _run_fused(n: int, gates, precision, split: bool = False, initial=None, reps
     st = Stream()
     e0, e1 = Event(), Event()
     ts = []
-    for rep in range(reps + (1 if warm else 0)):
+    untimed = (2 if use_graph else 1) if warm else 0  # the graph is captured at the second run
+    for rep in range(reps + untimed):
         if initial is None:
             sv.zero(st)
         else:
@@ -319,9 +335,9 @@ def _run_fused(n: int, gates, precision, split: bool = False, initial=None, reps
         prog.run(sv, st, use_graph=use_graph)
         e1.record(st)
         e1.sync()
-        if rep or not warm:
+        if rep >= untimed:
             ts.append(e1.elapsed_s(e0))
-    return float(np.median(ts)), sv
+    return float(np.median(ts)), sv, _passes(prog)
 
 
 def qft_leg(n: int = 22, seed: int = 7):
@@ -335,19 +351,19 @@ def qft_leg(n: int = 22, seed: int = 7):
     circ = QuantumCircuit.qft_cx(n)
     init = _random_state(n, seed)
     fused = optimize_native(n, circ.gates(), FusionConfig.default()).gates()
-    t, sv = _run_fused(n, fused, cu.CudaPrecision.F64, initial=init)
+    t, sv, passes = _run_fused(n, fused, cu.CudaPrecision.F64, initial=init)
     got = sv.download()
-    _, sv_u = _run_fused(n, circ.gates(), cu.CudaPrecision.F64, initial=init, reps=1)
+    _, sv_u, _ = _run_fused(n, circ.gates(), cu.CudaPrecision.F64, initial=init, reps=1)
     ref = sv_u.download()
-    passes = len(fused)
     from collections import Counter
 
     from cast_simulator_b200.simulator import gate_engine
 
     engines = Counter(gate_engine(g.matrix(), g.qubits(), n, cu.CudaPrecision.F64) for g in fused)
     return {"workload": f"qft-cx-{n}q-c128-default-fusion", "unfused_gates": len(circ),
-            "fused_gates": passes, "engines": dict(engines), "ms": t * 1e3,
-            "hbm_gbs": passes * 2 * (1 << n) * 16 / t / 1e9,
+            "fused_gates": len(fused), "engines": dict(engines), "ms": t * 1e3,
+            "note": "64 MiB state, resident in L2: the rates are not of HBM",
+            **{k.replace("hbm", "pass"): v for k, v in _program_rates(n, len(fused), passes, 16, t).items()},
             "gates_amps_per_s": len(circ) * (1 << n) / t,
             "max_abs_diff_vs_unfused": float(np.max(np.abs(got - ref)))}
 
@@ -379,14 +395,14 @@ def largest_leg(threads: int, depth: int = 10, n64: int = 34, n128: int = 33, n_
             base = None
             for k, split in variants:
                 fused = optimize_native(n, circ.gates(), FusionConfig.size_only(k)).gates()
-                t, sv = _run_fused(n, fused, prec, split, reps=1, warm=False, use_graph=False)
+                t, sv, passes = _run_fused(n, fused, prec, split, reps=1, warm=False, use_graph=False)
                 del sv
-                gbs = len(fused) * 2 * (1 << n) * amp / t / 1e9
+                rates = _program_rates(n, len(fused), passes, amp, t)
                 base = base or t
                 wl = f"{name}-{n}q" + (f"-d{depth}" if name == "brickwork" else "") + f"-{label}"
                 out["runs"].append({"workload": wl, "fusion_k": k,
                                     "tensor_cores": split, "fused_gates": len(fused), "ms": t * 1e3,
-                                    "hbm_gbs": gbs, "hbm_frac": gbs / peak,
+                                    **rates, "hbm_frac": rates["hbm_gbs"] / peak,
                                     "speedup_vs_plain_k4": base / t})
     fid = {}
     t0 = time.perf_counter()
@@ -399,7 +415,7 @@ def largest_leg(threads: int, depth: int = 10, n64: int = 34, n128: int = 33, n_
                                       ("c64-k5-tensor", cu.CudaPrecision.F32, 5, True),
                                       ("c64-k6-tensor", cu.CudaPrecision.F32, 6, True)):
             gk = g4 if k == 4 else optimize_native(n_prefix, circ.gates(), FusionConfig.size_only(k)).gates()
-            _, sv = _run_fused(n_prefix, gk, prec, split, reps=1, warm=False, use_graph=False)
+            _, sv, _ = _run_fused(n_prefix, gk, prec, split, reps=1, warm=False, use_graph=False)
             psi = sv.download()
             del sv
             fid[f"{name}-{label}"] = fidelity_vs(ref, psi)
@@ -491,12 +507,11 @@ def trajectory_leg(n: int = 16, depth: int = 30, n_traj: int = 4096, k: int = 3,
     idx = np.arange(1 << n)
     z_dm = np.array([1 - 2 * pops[(idx >> q) & 1 == 1].sum() for q in range(n)]) / pops.sum()
     dev = np.abs(mean - z_dm)
-    dm_passes = len(fused)
     out["density_matrix_exact"] = {
         "method": f"2n = {2 * n} virtual qubits, complex64 ({(8 << (2 * n)) / 2**30:.0f} GiB), "
                   "superoperators fused at k=4 on the plain kernels",
-        "fused_passes": dm_passes, "seconds": t_dm,
-        "hbm_gbs": dm_passes * 2 * (8 << (2 * n)) / t_dm / 1e9,
+        "fused_gates": len(fused), "seconds": t_dm,
+        **_program_rates(2 * n, len(fused), _passes(gp), 8, t_dm),
         "trajectory_mean_max_dev": float(dev.max()),
         "trajectory_mean_max_dev_in_stderr": float((dev / se).max())}
     # time to solution at a target standard error eps of every <Z_q>:
@@ -522,7 +537,7 @@ def sampling_leg(n: int = 30, depth: int = 20, n_shots: int = 1_000_000, k: int 
     import torch
 
     _, gates = build_fused(n, depth, k)
-    _, sv = _run_fused(n, gates, cu.CudaPrecision.F64, reps=1, warm=False, use_graph=False)
+    _, sv, _ = _run_fused(n, gates, cu.CudaPrecision.F64, reps=1, warm=False, use_graph=False)
     st = Stream()
     sample(sv, 1000, seed=1, stream=st)  # first launches
     # the keys land in one reused page-locked buffer: a direct DMA, no driver staging
@@ -692,8 +707,8 @@ def circuit_batch_leg(n_circ: int = 2048, n_range=(10, 16), depth_range=(5, 40),
 def fusion_sweep_leg(n: int, depth: int):
     """The brickwork with fusion width k = 2..7 on the CUDA-core path in complex128
     and complex64, and on the split-BF16 tensor cores for k = 5, 6 (complex64):
-    device time per circuit (median of 2 after a warm-up run), fused passes, and
-    the HBM rate those passes imply."""
+    device time per circuit (median of 2 after the warm-up runs), the passes a
+    program makes of the fused gates, and the HBM rate those imply."""
     from cast_simulator_b200 import cuda as cu
     from cast_simulator_b200.fusion import FusionConfig, optimize_native
     from cast_simulator_b200.types import QuantumCircuit
@@ -707,12 +722,12 @@ def fusion_sweep_leg(n: int, depth: int):
     fused = {k: optimize_native(n, circ.gates(), FusionConfig.size_only(k)).gates() for k in range(2, 8)}
     for prec, label, split, k in cases:
         gates = fused[k]
-        t, sv = _run_fused(n, gates, prec, split, reps=2)
+        t, sv, passes = _run_fused(n, gates, prec, split, reps=2)
         b_amp = 16 if label == "c128" else 8
-        gbs = len(gates) * 2 * (1 << n) * b_amp / t / 1e9
+        rates = _program_rates(n, len(gates), passes, b_amp, t)
         out["runs"].append({"precision": label, "tensor_cores": split, "fusion_k": k,
                             "fused_gates": len(gates), "ms_per_circuit": t * 1e3,
-                            "hbm_gbs": gbs, "hbm_frac": gbs / peak})
+                            **rates, "hbm_frac": rates["hbm_gbs"] / peak})
         del sv
     for label in ("c128", "c64"):
         best = min((r for r in out["runs"] if r["precision"] == label),
@@ -743,8 +758,8 @@ def tensor_leg(n: int, depth: int, sweep: dict):
         r = by_k[k]
         t = r["ms_per_circuit"] / 1e3
         run = {"fusion_k": k, "tensor_cores": r["tensor_cores"], "fused_gates": r["fused_gates"],
-               "ms_per_circuit": r["ms_per_circuit"], "hbm_gbs": r["hbm_gbs"],
-               "hbm_frac": r["hbm_gbs"] / peak}
+               "ms_per_circuit": r["ms_per_circuit"], "state_passes": r["state_passes"],
+               "gate_gbs": r["gate_gbs"], "hbm_gbs": r["hbm_gbs"], "hbm_frac": r["hbm_gbs"] / peak}
         if r["tensor_cores"]:
             gates = optimize_native(n, circ.gates(), FusionConfig.size_only(k)).gates()
             # tensor-pipe work of the passes that ran there: 3 split products of the
@@ -765,7 +780,7 @@ def tensor_leg(n: int, depth: int, sweep: dict):
     fid = {}
     for k in (5, 6):
         g = optimize_native(nf, small.gates(), FusionConfig.size_only(k)).gates()
-        _, sv = _run_fused(nf, g, cu.CudaPrecision.F32, True, reps=1, warm=False)
+        _, sv, _ = _run_fused(nf, g, cu.CudaPrecision.F32, True, reps=1, warm=False)
         fid[f"k{k}"] = fidelity_vs(ref, sv.download())
         del sv
     out["fidelity_24q_vs_cpu_fp64"] = fid
@@ -1031,6 +1046,7 @@ def main(argv=None):
         pg.all_reduce(et, op=pg.ReduceOp.MAX)
         e2e_t = float(et.item())
     e2e_value = ws * args.steps * len(gates) * bytes_per_pass / e2e_t / 1e9
+    e2e_passes = _passes(sim.compile_batch(gates, n))
 
     line = {
         "metric": "HBM GB/s (fused-gate statevector passes)",
@@ -1056,7 +1072,8 @@ def main(argv=None):
         "gates_amps_per_s": ws * args.steps * len(gates) * (1 << n) / t,
         "roofline": roofline_of(run, n, args.precision),
         "e2e": {"value": e2e_value, "unit": "GB/s", "h2d_bytes_per_step": h2d,
-                "d2h_bytes_per_step": d2h},
+                "d2h_bytes_per_step": d2h, "passes_per_step": e2e_passes,
+                "hbm_gbs": ws * args.steps * e2e_passes * bytes_per_pass / e2e_t / 1e9},
         "gpu_launches": run["n_launch"],
         "clocks": run["clocks"],
         "wall_s_timed": run["wall"],

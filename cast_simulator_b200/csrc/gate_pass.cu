@@ -1,5 +1,6 @@
 // Merged gate passes: several gates of a program applied to the statevector for
-// one read and one write of it (complex128, k <= 4).
+// one read and one write of it: dense gates of up to 4 qubits and sparse ones of 5
+// to 7, in both precisions.  complex128 first, complex64 below.
 //
 // A CTA owns a tile: the 2^tb amplitudes whose non-tile qubits are fixed
 // (pass_plan.hpp chooses the tile's qubits and its gates).  The tile is copied to
