@@ -99,14 +99,14 @@ __global__ void __launch_bounds__(kPassThreads, 3)
 
 // ── complex64 ────────────────────────────────────────────────────────────────
 //
-// The same passes in FP32, bound by the FP32 pipe: 24 packed pair FMAs
+// The same passes in FP32, bound by the FP32 pipe (59% busy) and shared memory
+// (78 to 86% of its wavefronts): 24 packed pair FMAs
 // (__ffma2_rn, two rows at once) an amplitude and 4-qubit gate.  A thread takes U
 // gather groups and, of a 4-qubit gate, half the rows (its partner for the other
 // half is in the same warp and reads the same amplitudes: a broadcast).  It walks
 // the columns with all its sums in registers; per column it reads U amplitudes
 // from the tile and its rows of the matrix, staged in shared memory one gate
-// ahead, at addresses the lanes share.  The FMA pipe is 59% busy (register
-// operands: three 64-bit reads a packed FMA); whole rows of two groups a thread
+// ahead, at addresses the lanes share.  Whole rows of two groups a thread
 // with the matrix read through L1 ran at 0.71 of this (28 qubits, fused at 4:
 // 64.3 against 46.8 ms; one gate a pass 56.0).  30 qubits, complex64, depth 20,
 // fused at 4: 232 -> 200 ms; 26 qubits fused at 3: 21.4 -> 12.3 ms, at 2: 40.4 ->
@@ -381,14 +381,20 @@ bool upload_pass_plan(PassPlan &p, std::string &err) {
   if (p.copies.on(dev)) return true;
   const void *src = p.pool.empty() ? (const void *)p.pool32.data() : (const void *)p.pool.data();
   RelaxedCapture relaxed;
-  // the shared-memory limit is a kernel's on one device
+  // the shared-memory limit is a kernel's on one device; tiles that launch without
+  // raising it do not wait for the calls
   auto opt_in = [&](auto kernel, size_t most) {
     return cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most),
                    "cudaFuncSetAttribute(gate pass kernel)", err);
   };
-  const size_t most64 = sizeof(double2) << kPassMaxTile, most32 = 2 * kPass32MatBytes + (sizeof(float2) << kPass32MaxTile);
-  if (p.pool.empty() ? !opt_in(k_gate_pass32<false>, most32) || !opt_in(k_gate_pass32<true>, most32)
-                     : !opt_in(k_gate_pass<false>, most64) || !opt_in(k_gate_pass<true>, most64))
+  constexpr size_t most64 = sizeof(double2) << kPassMaxTile;
+  constexpr size_t most32 = 2 * kPass32MatBytes + (sizeof(float2) << kPass32MaxTile);
+  size_t most = 0;
+  for (const PassArgs &a : p.args) most = std::max(most, sizeof(double2) << a.tb);
+  for (const PassArgs32 &a : p.args32) most = std::max(most, 2 * kPass32MatBytes + (sizeof(float2) << a.tb));
+  if (most > 48 * 1024 &&
+      (p.pool.empty() ? !opt_in(k_gate_pass32<false>, most32) || !opt_in(k_gate_pass32<true>, most32)
+                      : !opt_in(k_gate_pass<false>, most64) || !opt_in(k_gate_pass<true>, most64)))
     return false;
   PlanApi api{err};
   PlanBuffer<PlanApi> b;

@@ -381,14 +381,15 @@ __device__ __forceinline__ void pass_gate32(float2 *s, const float *mat, const P
   static_assert(GT == 1u << TB, "a power of two of groups");
   const uint32_t half = H == 2 ? (threadIdx.x >> 4) & 1 : 0;
   const uint32_t gt = H == 2 ? (threadIdx.x & 15) | (threadIdx.x >> 5) << 4 : threadIdx.x;
+  constexpr int LAST = (int)kTileMax32 - K;  // group bits of the largest tile
   auto offset = [&](uint32_t group, int from, int to) {  // group bits from .. to - 1
     uint32_t o = 0;
 #pragma unroll
-    for (int b = 0; b < (int)kTileMax32 - 1; ++b)
+    for (int b = 0; b < LAST; ++b)
       if (b >= from && b < to && ((group >> b) & 1)) o ^= g.group[b];
     return o;
   };
-  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0, LAST = (int)kTileMax32 - 1;
+  constexpr int LU = U == 4 ? 2 : U == 2 ? 1 : 0;
   static_assert(U == 1 << LU, "a power of two of groups");
   const uint32_t groups = 1u << (tb - K), t = offset(gt, 0, TB);
   if (groups >= U * GT) {

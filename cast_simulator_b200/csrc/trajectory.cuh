@@ -474,7 +474,7 @@ struct Traj {
   // and a matrix entry from shared memory for every four FMAs: 27 us a block of a
   // 16-qubit state, whose arithmetic takes 4 to 9.  2048 trajectories of 16 qubits and
   // depth 30 (fused at 3): 87.5 -> 73 ms; 18 qubits, depth 20 (296): 54 -> 37 ms; 12
-  // qubits (2048): 5.8 -> 4.8 ms.  What is left is latency: 16 warps issue 0.41
+  // qubits (2048): 5.8 -> 4.8 ms.  What is left is latency: 16 warps issue 0.45
   // instructions a clock and scheduler, waiting for shared memory and for each other.
   // The first applies the pending diagonal as its tiles
   // arrive, the last sums t and d (as gate_pass does) as its tiles leave.  Two tile
