@@ -9,10 +9,10 @@
 //    complex64 statevector lives in a per-CTA slice of a workspace in global
 //    memory (148 CTAs x 512 KiB = 74 MiB at 16 qubits, resident in the 126 MB
 //    L2); the CTA loops over trajectories blockIdx.x, blockIdx.x + gridDim.x, ...
-//  * GATE ops are fused unitary blocks (k <= 4).  A run of them up to the next DAMP
-//    or CHAN op is a segment: when none of its ERR sites fires (their draws do not
-//    depend on the state), its blocks share passes over the state as a gate
-//    program's gates do (pass_plan.hpp, gate_tile.cuh), tiles of up to 2^13
+//  * GATE ops are fused unitary blocks (k <= 4).  Pieces of a run of them up to the
+//    next DAMP or CHAN op are segments (seg_plan.cpp): when none of a segment's ERR
+//    sites fires (their draws do not depend on the state), its blocks share passes as
+//    a gate program's gates do (pass_plan.hpp, gate_tile.cuh), tiles of up to 2^13
 //    amplitudes in shared memory with the next tile's copy in flight; otherwise, and
 //    for programs without such segments, the blocks are applied one after the other
 //    in place;
@@ -141,10 +141,9 @@ __device__ __forceinline__ float2 cmul_add(float2 m, float2 x, float2 acc) {
 constexpr uint32_t kSegArgBytes = (cb2::kMaxPassGates * sizeof(cb2::PassGateArgs32) + 15) & ~15u;
 
 // The device side of one trajectory, for CTAs of NT threads.  512-thread CTAs
-// get 128 registers a thread, so the fused gates run without spills (the passes
-// of small and HBM-sized states are bound by instruction issue); 1024-thread
-// CTAs keep twice the loads in flight, which is what the L2-resident states of
-// 15 to 17 qubits need.
+// get 128 registers a thread, so the fused gates run without spills (their passes
+// are bound by instruction issue); 1024-thread CTAs keep twice the loads in flight,
+// which is what narrow blocks need on L2-resident states (plain_threads, seg_plan.cpp).
 template <int NT>
 struct Traj {
   static constexpr int kTThreads = NT;

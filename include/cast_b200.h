@@ -100,10 +100,11 @@ int cast_b200_gate_engine(uint8_t precision, uint32_t sv_n_qubits, const cast_co
  * compile_batch + apply-all + sync loop (src/simulator/mod.rs:523-562,
  * src/simulator/bench.rs:136-167).  With use_graph != 0 the launches are
  * captured into a CUDA graph at the second run on a (statevector, stream) pair
- * and replayed from then on.  Neighbouring dense gates of up to 4 qubits may
- * share one pass over the state (gates that share a qubit keep their order,
- * gates on disjoint qubits may swap); on a stream under capture by the caller,
- * and while a kernel choice is forced, every gate runs on its own kernel. */
+ * and replayed from then on.  Neighbouring gates (dense ones of up to 4 qubits,
+ * sparse ones of 5 to 7) may share one pass over the state: gates that share a
+ * qubit keep their order, gates on disjoint qubits may swap.  On a stream under
+ * capture by the caller every gate runs on its own kernel, and so do gates whose
+ * kernel is forced. */
 void *cast_b200_program_create(uint8_t precision, uint32_t sv_n_qubits, double ztol, double otol,
                                char *err_buf, size_t err_buf_len);
 int cast_b200_program_add_gate(void *program, const cast_complex64_t *matrix,
@@ -286,7 +287,7 @@ int cast_b200_traj_get_op(const void *program, uint32_t index, uint32_t *out_typ
                           uint32_t *out_n_mats, cast_complex64_t *out_mats, size_t out_mats_len);
 /* Launch shape of the trajectory kernel, a tuning knob with no counterpart in
  * the reference.  threads: threads per CTA, 512 or 1024, or 0 (the default) to
- * choose by state size.  max_ctas: CTAs, i.e. trajectories in flight (each owns
+ * choose by state and block size; a program given 1024 runs block by block.  max_ctas: CTAs, i.e. trajectories in flight (each owns
  * a 2^n-amplitude slice of the workspace), or 0 (the default) for one per SM. */
 int cast_b200_traj_set_launch(void *program, uint32_t threads, uint32_t max_ctas, char *err_buf,
                               size_t err_buf_len);
