@@ -152,6 +152,14 @@ struct Scratch {
 Scratch g_scratch_dev[kMaxScratchDevices];
 
 Scratch *ensure_scratch(int len, cudaStream_t stream, std::string &err) {
+  // a reduction waits for its result, which a stream under capture cannot give; said
+  // before anything is enqueued, it leaves the caller's capture (and this scratch) valid
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (!cuda_ok(cudaStreamIsCapturing(stream, &capturing), "cudaStreamIsCapturing (reduction)", err)) return nullptr;
+  if (capturing != cudaStreamCaptureStatusNone) {
+    err = "a reduction cannot run on a stream that is being captured";
+    return nullptr;
+  }
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice", err)) return nullptr;
   if (dev < 0 || dev >= kMaxScratchDevices) {

@@ -88,3 +88,31 @@ def test_reductions_on_many_streams_between_refusals(cblib):
     for t in threads:
         t.join()
     assert not wrong, wrong[:4]
+
+
+def test_a_reduction_refuses_a_stream_under_capture(cblib):
+    """Refused before anything is enqueued: the capture goes on and later reductions
+    keep their scratch."""
+    import torch
+
+    from cast_simulator_b200 import simulator as S
+    from cast_simulator_b200.cuda import CudaPrecision, CudaStatevector
+
+    sv = CudaStatevector(14, CudaPrecision.F64)
+    sv.zero()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    x = torch.zeros(8, device="cuda")
+
+    class Captured:
+        handle = side.cuda_stream
+
+    with torch.cuda.graph(graph, stream=side):
+        x += 1
+        with pytest.raises(RuntimeError, match="captured"):
+            S.qubit_populations(sv, Captured)
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8
+    p, norm = S.qubit_populations(sv, S.Stream())
+    assert norm == 1 and not p.any()
