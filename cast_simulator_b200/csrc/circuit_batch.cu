@@ -68,7 +68,7 @@ struct BCircuit {
 };
 
 struct alignas(16) BOp {
-  uint32_t mat;  // byte offset of the matrix in the pool (16-byte aligned)
+  uint32_t mat;  // where the matrix starts in the pool, in units of 16 bytes
   uint32_t mat_bytes;
   uint32_t k;
   uint32_t q[kBatchMaxGate];
@@ -217,7 +217,7 @@ __device__ void run_streamed(BShared &S, unsigned char *smem, const BOp *__restr
   V *Msm = reinterpret_cast<V *>(smem);
   for (uint32_t oi = 0; oi < c.n_ops; ++oi) {
     const BOp &op = ops[c.op_begin + oi];
-    const V *Mg = reinterpret_cast<const V *>(pool + op.mat);
+    const V *Mg = reinterpret_cast<const V *>(pool + (size_t)op.mat * 16);
     const uint32_t k = op.k, entries = 1u << (2 * k);
     for (uint32_t i = threadIdx.x; i < entries; i += NT) Msm[i] = Mg[i];
     __syncthreads();
@@ -258,7 +258,7 @@ __device__ void run_resident(BShared &S, unsigned char *smem, const BOp *__restr
   auto fetch = [&](uint32_t i, uint2 where) {
     unsigned char *to = smem + (i & 1) * kBMatBytes;
     for (uint32_t b = 16 * threadIdx.x; b < where.y; b += 16 * NT)
-      __pipeline_memcpy_async(to + b, pool + where.x + b, 16);
+      __pipeline_memcpy_async(to + b, pool + (size_t)where.x * 16 + b, 16);
     if (threadIdx.x < sizeof(BOp) / 16)
       __pipeline_memcpy_async(reinterpret_cast<char *>(&slots[i & 1]) + 16 * threadIdx.x,
                               reinterpret_cast<const char *>(op + i) + 16 * threadIdx.x, 16);
@@ -333,7 +333,8 @@ struct Batch {
   std::mutex mu;
   std::vector<BCircuit> circs;
   std::vector<BOp> ops;
-  std::vector<char> pool;   // matrices, each 16-byte aligned
+  std::vector<char> pool;   // matrices as the kernel reads them, each 16-byte aligned
+  size_t matrix_bytes = 0;  // of the gates' matrices by themselves: what the limit is on
   std::vector<uint64_t> cost;  // work estimate per circuit (ordering)
   std::vector<char> tables;    // header, circuits and ops of the last upload
   uint32_t n_z = 0;
@@ -361,12 +362,13 @@ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 // Takes back what a refused circuit has appended.
 struct Appended {
   Batch &b;
-  const size_t ops = b.ops.size(), pool = b.pool.size();
+  const size_t ops = b.ops.size(), pool = b.pool.size(), matrices = b.matrix_bytes;
   bool keep = false;
   ~Appended() {
     if (keep) return;
     b.ops.resize(ops);
     b.pool.resize(pool);
+    b.matrix_bytes = matrices;
   }
 };
 
@@ -429,6 +431,11 @@ bool add_circuit(Batch &b, uint64_t sv, uint32_t n, uint8_t prec, uint32_t n_gat
     const size_t entries = 1ull << (2 * k);
     cb2::snap_matrix(g, m, ztol, otol);
     size_t bytes = entries * (prec ? 16 : 8);
+    if (b.matrix_bytes + bytes > 0xFFFFFFF0ull) {
+      err = "batch matrix pool exceeds 4 GiB";
+      return false;
+    }
+    b.matrix_bytes += bytes;
     const void *from = prec ? (const void *)g.m64.data() : (const void *)g.m32.data();
     if (c.resident) {
       const cb2::PlacedGate placed = cb2::place_gate(g, tile_qubits);
@@ -440,11 +447,7 @@ bool add_circuit(Batch &b, uint64_t sv, uint32_t n, uint8_t prec, uint32_t n_gat
       from = prec ? (const void *)frag64.data() : (const void *)frag32.data();
     }
     static_assert(sizeof(float2) * 4 % 16 == 0, "the smallest matrix keeps the pool 16-byte aligned");
-    if (b.pool.size() + bytes > 0xFFFFFFF0ull) {
-      err = "batch matrix pool exceeds 4 GiB";
-      return false;
-    }
-    op.mat = (uint32_t)b.pool.size();
+    op.mat = (uint32_t)(b.pool.size() / 16);  // laid out, at most 1.5 times 4 GiB
     op.mat_bytes = (uint32_t)bytes;
     const char *const at = static_cast<const char *>(from);
     b.uploaded = false;
@@ -687,6 +690,7 @@ void cast_b200_batch_clear(void *batch) {
   b->circs.clear();
   b->ops.clear();
   b->pool.clear();
+  b->matrix_bytes = 0;
   b->cost.clear();
   b->uploaded = false;
   b->n_z = 0;
