@@ -184,6 +184,14 @@ __global__ void __launch_bounds__(kPassThreads, 3)
 
 // ── host side ────────────────────────────────────────────────────────────────
 
+// Allocating, freeing and copying on a private stream is safe while a stream is
+// captured; say so, or the capture would refuse it (and be invalid from then on).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The runtime calls behind plan_buffers.hpp; a call that fails says why in `err`.
 struct PlanApi {
   using Event = cudaEvent_t;
@@ -201,7 +209,10 @@ struct PlanApi {
   bool allocate(size_t bytes, char *&p) {
     return cuda_ok(cudaMalloc((void **)&p, bytes), "cudaMalloc (gate pass matrices)", err);
   }
-  void release(char *p) { cudaFree(p); }
+  void release(char *p) {
+    RelaxedCapture relaxed;  // a program may be dropped at any time
+    cudaFree(p);
+  }
 };
 
 PlanBufferPool<PlanApi> &buffer_pool() {
@@ -229,14 +240,6 @@ bool upload_now(void *dst, const void *src, size_t bytes, std::string &err) {
                  "cudaMemcpyAsync (gate pass matrices)", err) &&
          cuda_ok(cudaStreamSynchronize(s), "cudaStreamSynchronize (gate pass matrices)", err);
 }
-
-// Allocating and copying on a private stream is safe while another thread
-// captures; say so, or that thread's capture would refuse it.
-struct RelaxedCapture {
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 
 }  // namespace
 

@@ -116,3 +116,32 @@ def test_a_reduction_refuses_a_stream_under_capture(cblib):
     assert x.tolist() == [2.0] * 8
     p, norm = S.qubit_populations(sv, S.Stream())
     assert norm == 1 and not p.any()
+
+
+def test_dropping_a_large_program_leaves_a_capture_valid(cblib):
+    """A plan's buffer beyond what the pool keeps is freed at once, also while a stream
+    is being captured."""
+    import torch
+
+    from cast_simulator_b200 import simulator as S
+    from cast_simulator_b200.cuda import CudaPrecision, CudaStatevector
+    from cast_simulator_b200.types import QuantumGate
+
+    n, st = 12, S.Stream()
+    m = QuantumGate.random_unitary([0, 1, 2, 3], np.random.default_rng(0)).matrix()
+    prog = S.GateProgram(CudaPrecision.F64, n, 0.0, 0.0)
+    for i in range(11500):  # 6 KB of matrix each in the plan: more than 64 MB
+        prog.add(m, [i % 8, i % 8 + 1, i % 8 + 2, i % 8 + 3])
+    sv = CudaStatevector(n, CudaPrecision.F64)
+    sv.zero()
+    prog.run(sv, st)
+    st.sync()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    x = torch.zeros(8, device="cuda")
+    with torch.cuda.graph(graph, stream=side):
+        x += 1
+        del prog
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [2.0] * 8
