@@ -107,8 +107,9 @@ __device__ __forceinline__ uint64_t block_exclusive_scan(uint64_t v, uint64_t *w
   return ex;
 }
 
-// Pass 1: integer and FP64 totals of one chunk.
-template <typename T>
+// Pass 1: integer and FP64 totals of one chunk.  FULL: chunks of 2^kMaxChunkBits
+// amplitudes, a thread's loads all in flight; smaller states run without that code.
+template <typename T, bool FULL>
 __global__ void __launch_bounds__(kSmpThreads) k_chunk_totals(const T *__restrict__ x, uint32_t cb,
                                                              double scale, uint64_t *__restrict__ qtot,
                                                              double *__restrict__ ptot) {
@@ -119,7 +120,7 @@ __global__ void __launch_bounds__(kSmpThreads) k_chunk_totals(const T *__restric
   const V *xv = reinterpret_cast<const V *>(x) + (chunk << cb);
   uint64_t q = 0;
   double p = 0.0;
-  if (cb == kMaxChunkBits) {  // a full chunk: every load of the thread in flight at once
+  if constexpr (FULL) {
     V v[kFullPer];
 #pragma unroll
     for (uint32_t u = 0; u < kFullPer; ++u) v[u] = xv[threadIdx.x + u * kSmpThreads];
@@ -300,7 +301,7 @@ __global__ void k_chunk_first_shot(const uint64_t *__restrict__ start, uint64_t 
 }
 
 // Pass 3.
-template <typename T>
+template <typename T, bool FULL>
 __global__ void __launch_bounds__(kSmpThreads) k_sample_assign(
     const T *__restrict__ x, uint32_t cb, const uint64_t *__restrict__ start,
     const uint64_t *__restrict__ first, Targets tg, double scale,
@@ -319,7 +320,7 @@ __global__ void __launch_bounds__(kSmpThreads) k_sample_assign(
   const uint32_t nt = c < (uint32_t)kSmpThreads ? c : (uint32_t)kSmpThreads;
   const uint32_t per = c / nt;
   const V *xv = reinterpret_cast<const V *>(x) + (chunk << cb);
-  if (cb == kMaxChunkBits) {
+  if constexpr (FULL) {
     V v[kFullPer];
 #pragma unroll
     for (uint32_t u = 0; u < kFullPer; ++u) v[u] = xv[threadIdx.x + u * kSmpThreads];
@@ -438,12 +439,14 @@ bool sample_impl(const void *sv, uint32_t n, uint64_t n_shots, bool seeded, uint
   std::string e2;
   bool ok = true;
   double scale = kFix;
+  const bool full = cb == kMaxChunkBits;
   // A normalised state takes one pass with no host round trip before the final
   // copy: the totals, scans, status check, searches and assignment are queued
   // back to back and the host reads the status with the keys.  Only a state
   // whose total is far from 1 takes a second pass, scaled by its true total.
   for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-    k_chunk_totals<T><<<(unsigned)n_chunks, kSmpThreads, 0, s>>>(x, cb, scale, qtot, ptot);
+    const auto totals = full ? k_chunk_totals<T, true> : k_chunk_totals<T, false>;
+    totals<<<(unsigned)n_chunks, kSmpThreads, 0, s>>>(x, cb, scale, qtot, ptot);
     k_sum_fp<<<1, kScanThreads, 0, s>>>(ptot, n_chunks, reinterpret_cast<double *>(grand + 2));
     k_scan_tiles<<<(unsigned)tiles_c, kScanThreads, 0, s>>>(qtot, n_chunks, tt_c);
     k_scan_small<<<1, kScanThreads, 0, s>>>(tt_c, tiles_c, grand);
@@ -464,8 +467,8 @@ bool sample_impl(const void *sv, uint32_t n, uint64_t n_shots, bool seeded, uint
     k_check<<<1, 32, 0, s>>>(grand, seeded ? 1 : 0, attempt == 0 ? 1 : 0);
     const unsigned fg = (unsigned)std::min<uint64_t>((n_chunks + 256) / 256, 16ull * sm_count());
     k_chunk_first_shot<<<fg, 256, 0, s>>>(start, n_chunks, tg, n_shots, first);
-    k_sample_assign<T><<<(unsigned)n_chunks, kSmpThreads, 0, s>>>(x, cb, start, first, tg, scale, km,
-                                                                   keys);
+    const auto assign = full ? k_sample_assign<T, true> : k_sample_assign<T, false>;
+    assign<<<(unsigned)n_chunks, kSmpThreads, 0, s>>>(x, cb, start, first, tg, scale, km, keys);
     uint64_t g[4] = {0, 0, 0, 0};
     ok = cuda_ok(cudaGetLastError(), "sampling launch", err) &&
          cuda_ok(cudaMemcpyAsync(host_out, keys, n_shots * 8, cudaMemcpyDeviceToHost, s),
